@@ -207,9 +207,11 @@ int opflow_batch_solve(opflow_batch b, opflow_solve_state* states) {
         ProblemHost& P = S->probs[p];
         const long long N = P.levels[0].N;
         const double sb = mg_sum(ctx, P.b, N);
-        OPG_CUDA(cudaMemcpy(&b_pin[p], P.b, 8, cudaMemcpyDeviceToHost));
+        OPG_CUDA(cudaMemcpyAsync(&b_pin[p], P.b, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
         const double nb0 = -(sb - b_pin[p]);
-        OPG_CUDA(cudaMemcpy(P.b, &nb0, 8, cudaMemcpyHostToDevice));
+        OPG_CUDA(cudaMemcpyAsync(P.b, &nb0, 8, cudaMemcpyHostToDevice, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     OPG_TRY(mg_solve(S));
     std::vector<Scal> st;
@@ -219,9 +221,11 @@ int opflow_batch_solve(opflow_batch b, opflow_solve_state* states) {
         ProblemHost& P = S->probs[p];
         const long long N = P.levels[0].N;
         double shift = 0.;
-        OPG_CUDA(cudaMemcpy(&shift, S->kd_host[p].x, 8, cudaMemcpyDeviceToHost));
+        OPG_CUDA(cudaMemcpyAsync(&shift, S->kd_host[p].x, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
         mg_add_scalar(ctx, S->kd_host[p].x, N, -shift);
-        OPG_CUDA(cudaMemcpy(P.b, &b_pin[p], 8, cudaMemcpyHostToDevice));
+        OPG_CUDA(cudaMemcpyAsync(P.b, &b_pin[p], 8, cudaMemcpyHostToDevice, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     // true residuals of every problem
     const int np = (int) S->probs.size();

@@ -177,9 +177,11 @@ static int setup_req(opflow_server S, Req* r, Scal* seed) {
         // the pinned system (first unknown held at 0): singular system with b[0] = -(sum of the others)
         const double sb = mg_sum(ctx, P.b, r->N);
         double b0 = 0.;
-        OPG_CUDA(cudaMemcpy(&b0, P.b, 8, cudaMemcpyDeviceToHost));
+        OPG_CUDA(cudaMemcpyAsync(&b0, P.b, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
         const double nb0 = -(sb - b0);
-        OPG_CUDA(cudaMemcpy(P.b, &nb0, 8, cudaMemcpyHostToDevice));
+        OPG_CUDA(cudaMemcpyAsync(P.b, &nb0, 8, cudaMemcpyHostToDevice, ctx->stream));
+        OPG_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     OPG_TRY(mg_prepare_problem(M, S->params.tol, M->dS));
     OPG_CUDA(cudaMemcpyAsync(seed, M->dS, sizeof(Scal), cudaMemcpyDeviceToHost, ctx->stream));

@@ -348,7 +348,10 @@ static int compress_level(MGSystem* S, LevelHost& L) {
 static int coarse_inverse(MGSystem* S, LevelHost& L, bool singular) {
     const int N = (int) L.N;
     std::vector<double> A((size_t) N * N, 0.), coefs((size_t) NSLOT * N);
-    OPG_CUDA(cudaMemcpy(coefs.data(), L.A64, coefs.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    // (copies on the context's stream: pool memory belongs to the stream it was allocated on, and a copy on
+    // another stream would not wait for what that stream still waits for)
+    OPG_CUDA(cudaMemcpyAsync(coefs.data(), L.A64, coefs.size() * sizeof(double), cudaMemcpyDeviceToHost, S->ctx->stream));
+    OPG_CUDA(cudaStreamSynchronize(S->ctx->stream));
     for (int c = 0; c < N; ++c) {
         const int i = c % L.n[0], j = (c / L.n[0]) % L.n[1], k = c / (L.n[0] * L.n[1]);
         const int idx[3] = {i, j, k};
@@ -401,7 +404,8 @@ static int coarse_inverse(MGSystem* S, LevelHost& L, bool singular) {
         for (int c = 0; c < M; ++c) Full[(size_t) (r + off) * N + (c + off)] = Inv[(size_t) r * M + c];
     L.Ainv64 = (double*) S->arena.alloc(Full.size() * sizeof(double));
     if (!L.Ainv64) return fail(OPFLOW_E_NOMEM, "coarse inverse");
-    OPG_CUDA(cudaMemcpy(L.Ainv64, Full.data(), Full.size() * sizeof(double), cudaMemcpyHostToDevice));
+    OPG_CUDA(cudaMemcpyAsync(L.Ainv64, Full.data(), Full.size() * sizeof(double), cudaMemcpyHostToDevice, S->ctx->stream));
+    OPG_CUDA(cudaStreamSynchronize(S->ctx->stream));
     return OPFLOW_OK;
 }
 
