@@ -252,17 +252,22 @@ __device__ __forceinline__ void cell_prolong(const LvlDev* __restrict__ Ls, cons
     Sel<T>::x(Lf)[cell_of(Lf, f0, f1, f2)] += acc;
 }
 
-// coarsest level: x = Ainv b (dense, accumulated in float64), rows t0, t0+dt, ...
+// coarsest level: x = Ainv b (dense, accumulated in float64), by all dt threads of a CTA (whole warps):
+// eight lanes share a row, so that a row's chain of dependent float64 operations is 1/8 as long
 template <typename T>
 __device__ __forceinline__ void coarse_rows(const LvlDev& L, int t0, int dt) {
     const T* b = Sel<T>::b(L);
     T* x = Sel<T>::x(L);
     const int N = (int) L.N;
-    for (int row = t0; row < N; row += dt) {
+    for (int base = 0; base < N; base += dt / 8) {
+        const int row = base + t0 / 8;
         double acc = 0.;
-        const double* Ar = L.Ainv64 + (long long) row * N;
-        for (int col = 0; col < N; ++col) acc = fma(Ar[col], (double) b[col], acc);
-        x[row] = (T) acc;
+        if (row < N) {
+            const double* Ar = L.Ainv64 + (long long) row * N;
+            for (int col = t0 & 7; col < N; col += 8) acc = fma(Ar[col], (double) b[col], acc);
+        }
+        for (int s = 4; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+        if (row < N && (t0 & 7) == 0) x[row] = (T) acc;
     }
 }
 

@@ -36,15 +36,18 @@ int mg_z_batch(int zb);
 int mg_launch_prolong_z(cudaStream_t s, int sms, bool f32, const LvlDev* L, const Chunk* ch, int nch, const Scal* sc, int zb);
 int mg_launch_restrict(cudaStream_t s, int sms, bool f32, const LvlDev* L, const Chunk* ch, int nch, const Scal* sc);
 int mg_launch_prolong(cudaStream_t s, int sms, bool f32, const LvlDev* L, const Chunk* ch, int nch, const Scal* sc);
-// fused 2D tile steps of a level (mg_tiles.cu): down = pre-smoothing + residual + restriction,
-// up = prolongation + post-smoothing; tiles are Chunk{lvl, j = tile y origin, k = 0, i0 = tile x origin}
-// 54 columns: with the down step's 5-cell halo a region row is 64 positions, one colour of it one
-// warp-wide pass; small levels use MG_TILE_X_SMALL x MG_TILE_Y / 2 (32-position rows)
-constexpr int MG_TILE_X = 54, MG_TILE_Y = 32, MG_TILE_X_SMALL = 22;
+// fused 2D steps of a float32 level (mg_tiles.cu): down = pre-smoothing from x = 0 + residual +
+// restriction, up = prolongation + post-smoothing; one warp per strip Chunk{lvl, j = first row, k = 0,
+// i0 = first column, cnt = columns, nrows = rows}, cut by mg_strips for `sweeps` = max(pre, post)
+constexpr int MG_STRIP_SWEEPS = 4;
 bool mg_tiles_supported(int sweeps);
-int mg_tiles_prepare(int sweeps);
-int mg_launch_tile_down(cudaStream_t s, int sms, bool f32, const LvlDev* L, const Chunk* tiles, int ntiles, const Scal* sc, int pre);
-int mg_launch_tile_up(cudaStream_t s, int sms, bool f32, const LvlDev* L, const Chunk* tiles, int ntiles, const Scal* sc, int post);
+void mg_strips(int li, const LvlDev& D, bool coarse_node, int sweeps, int rows, std::vector<Chunk>& out);
+int mg_launch_tile_down(cudaStream_t s, const LvlDev* L, const Chunk* strips, int n, const Scal* sc, int pre, int post);
+int mg_launch_tile_up(cudaStream_t s, const LvlDev* L, const Chunk* strips, int n, const Scal* sc, int pre, int post);
+// the V-cycle at and below each listed level of 2D problems whose levels there all take strips and whose
+// coarsest level has a dense inverse (pre = post = sweeps)
+constexpr int MG_BSTRIP_WARPS = 16, MG_BSTRIP_ROWS = 4;
+int mg_launch_bottom_strips(cudaStream_t s, const LvlDev* L, const int* top, int ntop, const Scal* sc, int sweeps);
 // the whole V-cycle below each listed level (a problem's first small level), one CTA per problem with
 // those levels' vectors in shared memory: at most MG_BOTTOM_LEVELS levels and MG_BOTTOM_CELLS cells
 // in all (`cells`: the largest such total of the listed problems)

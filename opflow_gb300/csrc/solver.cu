@@ -334,6 +334,17 @@ static int compress_level(MGSystem* S, LevelHost& L) {
     L.T32 = dt8f;
     L.table = hb == 0;
     L.tab = tab;
+    // (the float32 values decide: the strips that use it run the float32 V-cycle)
+    L.uoff = L.table && L.ndim == 2;
+    for (int cls = 0; L.uoff && cls < 9; ++cls) {
+        const int c[2] = {cls % 3, cls / 3};
+        for (int d = 0; d < 2; ++d)
+            for (int sd = 0; sd < 2; ++sd) {
+                const int q = 1 + 2 * d + sd;
+                const bool exists = L.per[d] || c[d] != (sd ? 2 : 0);
+                if (exists && t8f[cls * TSTRIDE + q] != t8f[4 * TSTRIDE + q]) L.uoff = false;
+            }
+    }
     if (!L.table) {
         L.A32 = (float*) S->arena.alloc((size_t) NSLOT * N * sizeof(float));
         if (!L.A32) return fail(OPFLOW_E_NOMEM, "float32 operator");
@@ -597,7 +608,6 @@ static int tune_levels(MGSystem* S) {
     for (int l = 0; l < S->nlevels; ++l) any = any || S->d_zsm[l].n > 0 || !S->tile_alt[l].empty();
     if (!any) return OPFLOW_OK;
     opflow_ctx ctx = S->ctx;
-    const int sms = ctx->num_sms;
     const bool f32 = S->precision == OPFLOW_PREC_MIXED;
     const size_t es = f32 ? 4 : 8;
     auto choose = [&](const std::string& key, const std::vector<int>& cands, const std::function<float(int)>& time_ms) {
@@ -633,8 +643,8 @@ static int tune_levels(MGSystem* S) {
                 }
                 const ChunkList& T = cand ? alt : S->d_tiles[l];
                 return time_launch(S, [&] {
-                    OPG_TRY(mg_launch_tile_down(ctx->stream, sms, f32, S->dL, T.ptr, T.n, nullptr, S->pre));
-                    return mg_launch_tile_up(ctx->stream, sms, f32, S->dL, T.ptr, T.n, nullptr, S->post);
+                    OPG_TRY(mg_launch_tile_down(ctx->stream, S->dL, T.ptr, T.n, nullptr, S->pre, S->post));
+                    return mg_launch_tile_up(ctx->stream, S->dL, T.ptr, T.n, nullptr, S->pre, S->post);
                 });
             });
             if (pick == 1) {
@@ -673,12 +683,12 @@ int mg_finalize(MGSystem* S) {
     S->coarse_sm_ch.clear();
     S->bottom_host.clear();
     S->bottom_cells_host.clear();
+    S->bstrip_host.clear();
     OPG_TRY(mg_bottom_prepare());
     const char* te = getenv("OPFLOW_MG_TILES");
-    // tiles for the float32 V-cycle only: the float64 one is bound by float64 issue, where the halo's
+    // strips for the float32 V-cycle only: the float64 one is bound by float64 issue, where the halo's
     // repeated sweeps cost more than the saved passes over memory (measured)
     bool tiles_on = f32 && !(te && te[0] == '0') && mg_tiles_supported(S->pre) && mg_tiles_supported(S->post);
-    if (tiles_on) OPG_TRY(mg_tiles_prepare(std::max(S->pre, S->post)));
     const char* ze = getenv("OPFLOW_MG_ZMARCH");
     const bool zoff = ze && ze[0] == '0';
     std::vector<int> coarse_list;
@@ -705,7 +715,7 @@ int mg_finalize(MGSystem* S) {
                 out.push_back(c);
             }
     };
-    if (const char* e = getenv("OPFLOW_MG_BOTTOM")) S->bottom_max = atoll(e);
+    if (const char* e = getenv("OPFLOW_MG_BOTTOM")) S->bottom_max = S->bstrip_max = atoll(e);
     // level-0 chunks of the Krylov kernels: whole rows of one plane, about KCH cells each (rows longer
     // than KCH are split), so the per-chunk reduction and its barriers are amortised over many cells.
     // KCH is 8192 for problems of at least 8192 cells per two SMs and halves (down to 1024) for smaller
@@ -730,25 +740,35 @@ int mg_finalize(MGSystem* S) {
                 out.push_back(c);
             }
     };
+    // Rows of a strip of the 2D levels at depth l (of every problem there): the most that still gives
+    // STRIP_FILL strips per SM.  Tall strips recompute fewer halo rows, short ones keep more warps on a
+    // small level, where a step takes as long as one strip's march.  2048^2 solve / batch of 64 Helmholtz
+    // problems (18.5 M cells) with 4, 8, 16, 32 strips per SM: 4.43, 4.39, 4.33, 4.33 / 11.6, 11.3, 11.1,
+    // 10.9 ms.
+    auto strip_rows = [&](size_t l) {
+        const int STRIP_FILL = 32;
+        const int w = 64 - 4 * std::max(S->pre, S->post);
+        for (int rows = 64; rows > 8; rows /= 2) {
+            long long n = 0;
+            for (const ProblemHost& P : S->probs)
+                if (l < P.levels.size() && P.levels[l].ndim == 2)
+                    n += (long long) ((P.levels[l].n[0] + w - 1) / w) * ((P.levels[l].n[1] + rows - 1) / rows);
+            if (n >= (long long) STRIP_FILL * ctx->num_sms) return rows;
+        }
+        return 8;
+    };
     for (size_t p = 0; p < S->probs.size(); ++p) {
         ProblemHost& P = S->probs[p];
         const int base = (int) lv.size();
-        // first level small enough for the one-CTA bottom kernel (levels.size(): none)
-        size_t sp = P.levels.size();
-        for (size_t l = 0; l < P.levels.size(); ++l)
-            if (P.levels[l].N <= S->bottom_max) { sp = l; break; }
-        long long bcells = 0;
-        for (size_t l = sp; l < P.levels.size(); ++l) bcells += P.levels[l].N;
-        if (bcells > MG_BOTTOM_CELLS || P.levels.size() - sp > (size_t) MG_BOTTOM_LEVELS) sp = P.levels.size();  // chunked instead
-        // 2D red-black class-table levels above the bottom whose coarse cells all have children in the
-        // level run as fused tiles
-        auto tileable = [&](size_t l) {
-            if (!tiles_on || l >= sp || l + 1 >= P.levels.size()) return false;
+        // 2D red-black class-table levels whose coarse cells all have children in the level run as fused
+        // strips (a periodic level of at least twice a strip's reach in rows)
+        auto stripable = [&](size_t l) {
+            if (!tiles_on || l + 1 >= P.levels.size()) return false;
             const LevelHost& F = P.levels[l];
             const LevelHost& Cn = P.levels[l + 1];
             if (F.ndim != 2 || !F.table) return false;
             for (int d = 0; d < 2; ++d) {
-                if (F.per[d] && (F.n[d] & 1)) return false;  // damped Jacobi level
+                if (F.per[d] && ((F.n[d] & 1) || F.n[d] < 32)) return false;  // (odd: a damped Jacobi level)
                 if (Cn.node) {
                     if (2 * Cn.lo[d] - F.lo[d] < 0 || 2 * (Cn.lo[d] + Cn.n[d] - 1) - F.lo[d] > F.n[d] - 1) return false;
                 } else if (Cn.n[d] != (F.n[d] + 1) / 2) {
@@ -757,6 +777,22 @@ int mg_finalize(MGSystem* S) {
             }
             return true;
         };
+        // first level small enough for a one-CTA bottom kernel (levels.size(): none): the strips' where every
+        // level from there on takes them down to a dense coarsest solve, else the per-cell one
+        size_t sp = P.levels.size();
+        for (size_t l = 0; l < P.levels.size(); ++l)
+            if (P.levels[l].N <= S->bstrip_max) { sp = l; break; }
+        bool bstrip = S->pre == S->post && P.levels.back().Ainv64 && sp + 1 < P.levels.size() && (sp == 0 || stripable(sp - 1));
+        for (size_t l = sp; bstrip && l + 1 < P.levels.size(); ++l) bstrip = stripable(l) && P.levels[l].uoff;
+        long long bcells = 0;
+        if (!bstrip) {
+            sp = P.levels.size();
+            for (size_t l = 0; l < P.levels.size(); ++l)
+                if (P.levels[l].N <= S->bottom_max) { sp = l; break; }
+            for (size_t l = sp; l < P.levels.size(); ++l) bcells += P.levels[l].N;
+            if (bcells > MG_BOTTOM_CELLS || P.levels.size() - sp > (size_t) MG_BOTTOM_LEVELS) sp = P.levels.size();  // chunked instead
+        }
+        auto tileable = [&](size_t l) { return l < sp && stripable(l); };
         for (size_t l = 0; l < P.levels.size(); ++l) {
             LevelHost& H = P.levels[l];
             LvlDev D{};
@@ -771,6 +807,7 @@ int mg_finalize(MGSystem* S) {
             D.N = H.N;
             D.node = H.node;
             D.table = H.table;
+            D.uoff = H.uoff;
             bool odd_periodic = false;
             for (int d = 0; d < H.ndim; ++d) odd_periodic = odd_periodic || (H.per[d] && (H.n[d] & 1));
             D.rbgs = !odd_periodic;
@@ -799,27 +836,20 @@ int mg_finalize(MGSystem* S) {
             }
             lv.push_back(D);
             const int li = base + (int) l;
-            if (l == sp) {
+            if (l == sp && bstrip) {
+                S->bstrip_host.push_back(li);
+            } else if (l == sp) {
                 S->bottom_host.push_back(li);
                 S->bottom_cells_host.push_back(bcells);
             }
             if (l >= sp) continue;                                   // inside the bottom kernel
             const bool above_tiled = l > 0 && tileable(l - 1);      // restricted by the finer level's tiles
             if (D.tiled) {
-                // 54 x 32 tiles, or 22 x 16 where that would leave SMs idle (tile extent: cnt x nrows);
-                // a single-problem system also keeps the other shape for the tuner
-                const bool small = (long long) ((D.n[0] + MG_TILE_X - 1) / MG_TILE_X) * ((D.n[1] + MG_TILE_Y - 1) / MG_TILE_Y) < 2LL * ctx->num_sms;
-                auto tiles = [&](bool sm, std::vector<Chunk>& out) {
-                    const int tx = sm ? MG_TILE_X_SMALL : MG_TILE_X, ty = sm ? MG_TILE_Y / 2 : MG_TILE_Y;
-                    for (int j0 = 0; j0 < D.n[1]; j0 += ty)
-                        for (int i0 = 0; i0 < D.n[0]; i0 += tx) {
-                            Chunk c{li, j0, 0, i0, tx};
-                            c.nrows = ty;
-                            out.push_back(c);
-                        }
-                };
-                tiles(small, S->tile_ch[l]);
-                if (S->probs.size() == 1 && tune_enabled()) tiles(!small, S->tile_alt[l]);
+                const bool cnode = P.levels[l + 1].node;
+                const int rows = strip_rows(l);
+                mg_strips(li, D, cnode, std::max(S->pre, S->post), rows, S->tile_ch[l]);
+                if (S->probs.size() == 1 && tune_enabled())
+                    mg_strips(li, D, cnode, std::max(S->pre, S->post), rows > 16 ? rows / 2 : 2 * rows, S->tile_alt[l]);
             } else {
                 const bool zmarch = !zoff && D.ndim == 3 && D.table && D.rbgs && !D.coarsest && D.N >= MG_ZT_MIN && D.n[0] >= 3 && D.n[1] >= 3 &&
                                     D.n[2] >= 3;
@@ -916,8 +946,11 @@ int mg_finalize(MGSystem* S) {
     S->bottom_cells = 0;
     for (long long c : S->bottom_cells_host) S->bottom_cells = std::max(S->bottom_cells, c);
     S->dbottom = (int*) S->arena.alloc(std::max<size_t>(1, S->bottom_host.size()) * sizeof(int));
-    if (!S->dbottom) return fail(OPFLOW_E_NOMEM, "solver tables");
+    S->nbstrip = (int) S->bstrip_host.size();
+    S->dbstrip = (int*) S->arena.alloc(std::max<size_t>(1, S->bstrip_host.size()) * sizeof(int));
+    if (!S->dbottom || !S->dbstrip) return fail(OPFLOW_E_NOMEM, "solver tables");
     if (S->nbottom) cudaMemcpyAsync(S->dbottom, S->bottom_host.data(), S->bottom_host.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+    if (S->nbstrip) cudaMemcpyAsync(S->dbstrip, S->bstrip_host.data(), S->bstrip_host.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
     if (!S->dL || !S->dK || !S->dS || !S->dk0 || !S->partial || !S->red || !S->dcoarse) return fail(OPFLOW_E_NOMEM, "solver tables");
     cudaMemcpyAsync(S->dL, lv.data(), lv.size() * sizeof(LvlDev), cudaMemcpyHostToDevice, ctx->stream);
     cudaMemcpyAsync(S->dK, kd.data(), kd.size() * sizeof(KrylovDev), cudaMemcpyHostToDevice, ctx->stream);
@@ -992,7 +1025,7 @@ static int vcycle(MGSystem* S) {
     const Scal* sc = S->dS;
     for (int l = 0; l < S->nlevels; ++l) {
         if (l > 0) OPG_TRY(mg_launch_restrict(s, sms, f32, S->dL, S->d_restrict[l].ptr, S->d_restrict[l].n, sc));
-        OPG_TRY(mg_launch_tile_down(s, sms, f32, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->pre));
+        OPG_TRY(mg_launch_tile_down(s, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->pre, S->post));
         const ChunkList& C = S->d_smooth[l];
         const ChunkList& Z = S->d_zsm[l];
         for (int it = 0; it < S->pre; ++it) {
@@ -1004,6 +1037,7 @@ static int vcycle(MGSystem* S) {
         OPG_TRY(mg_launch_residual(s, sms, f32, S->dL, C.ptr, C.n, sc));
         OPG_TRY(mg_launch_residual_z(s, sms, f32, S->dL, Z.ptr, Z.n, sc, S->zb[l]));
     }
+    OPG_TRY(mg_launch_bottom_strips(s, S->dL, S->dbstrip, S->nbstrip, sc, S->pre));
     OPG_TRY(mg_launch_bottom(s, sms, f32, S->dL, S->dbottom, S->nbottom, sc, S->pre, S->post, S->bottom_cells));
     OPG_TRY(mg_launch_coarse(s, sms, f32, S->dL, S->dcoarse, S->ncoarse, sc));
     for (int it = 0; it < S->pre + S->post; ++it) {
@@ -1011,7 +1045,7 @@ static int vcycle(MGSystem* S) {
         OPG_TRY(mg_launch_smooth(s, sms, f32, S->dL, S->d_coarse_sm.ptr, S->d_coarse_sm.n, 1, sc));
     }
     for (int l = S->nlevels - 2; l >= 0; --l) {
-        OPG_TRY(mg_launch_tile_up(s, sms, f32, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->post));
+        OPG_TRY(mg_launch_tile_up(s, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->pre, S->post));
         const ChunkList& C = S->d_smooth[l];
         const ChunkList& Z = S->d_zsm[l];
         OPG_TRY(mg_launch_prolong(s, sms, f32, S->dL, S->d_prolong[l].ptr, S->d_prolong[l].n, sc));
@@ -1261,7 +1295,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     std::vector<LvlDev> lv;
     std::vector<KrylovDev> kd;
     std::vector<Chunk> k0;
-    std::vector<int> first, count, coarse_list, bottom_list;
+    std::vector<int> first, count, coarse_list, bottom_list, bstrip_list;
     std::vector<long long> bottom_cells;
     C->bottom_cells = 0;
     C->nlevels = 0;
@@ -1295,6 +1329,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
         }
         for (int c : P->coarse_host) coarse_list.push_back(base + c);
         for (int b : P->bottom_host) bottom_list.push_back(base + b);
+        for (int b : P->bstrip_host) bstrip_list.push_back(base + b);
         for (long long c : P->bottom_cells_host) {
             bottom_cells.push_back(c);
             C->bottom_cells = std::max(C->bottom_cells, c);
@@ -1341,11 +1376,14 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     C->bottom_cells_host = bottom_cells;
     C->nbottom = (int) bottom_list.size();
     C->dbottom = (int*) C->arena.alloc(std::max<size_t>(1, bottom_list.size()) * sizeof(int));
+    C->bstrip_host = bstrip_list;
+    C->nbstrip = (int) bstrip_list.size();
+    C->dbstrip = (int*) C->arena.alloc(std::max<size_t>(1, bstrip_list.size()) * sizeof(int));
     C->d_active = (int*) C->arena.alloc(2 * sizeof(int));
     C->d_done = (int*) C->arena.alloc(np * sizeof(int));
     if (!C->d_done) return fail(OPFLOW_E_NOMEM, "batch tables");
     cudaMemsetAsync(C->d_done, 0, np * sizeof(int), ctx->stream);
-    if (!C->dL || !C->dK || !C->dS || !C->dk0 || !C->dfirst || !C->dcount || !C->partial || !C->red || !C->dcoarse || !C->d_active || !C->dbottom)
+    if (!C->dL || !C->dK || !C->dS || !C->dk0 || !C->dfirst || !C->dcount || !C->partial || !C->red || !C->dcoarse || !C->d_active || !C->dbottom || !C->dbstrip)
         return fail(OPFLOW_E_NOMEM, "batch tables");
     cudaStream_t s = ctx->stream;
     if (!lv.empty()) cudaMemcpyAsync(C->dL, lv.data(), lv.size() * sizeof(LvlDev), cudaMemcpyHostToDevice, s);
@@ -1356,6 +1394,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     if (!count.empty()) cudaMemcpyAsync(C->dcount, count.data(), count.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (!coarse_list.empty()) cudaMemcpyAsync(C->dcoarse, coarse_list.data(), coarse_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (!bottom_list.empty()) cudaMemcpyAsync(C->dbottom, bottom_list.data(), bottom_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
+    if (!bstrip_list.empty()) cudaMemcpyAsync(C->dbstrip, bstrip_list.data(), bstrip_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     auto upload = [&](std::vector<Chunk>& h, ChunkList& d) {
         d.n = (int) h.size();
         d.ptr = (Chunk*) C->arena.alloc(std::max<size_t>(1, h.size()) * sizeof(Chunk));

@@ -26,6 +26,7 @@ struct LevelHost {
     int per[3] = {0, 0, 0};
     int gh_lo[3] = {GH_COPY, GH_COPY, GH_COPY}, gh_hi[3] = {GH_COPY, GH_COPY, GH_COPY};
     bool table = false;
+    bool uoff = false;  // LvlDev::uoff
     std::vector<double> tab;
     double* A64 = nullptr;
     float* A32 = nullptr;
@@ -103,6 +104,13 @@ struct MGSystem {
     std::vector<int> coarse_host, bottom_host;
     int* dbottom = nullptr;
     int nbottom = 0;
+    // 2D problems whose small levels all take strips: their first level of at most bstrip_max cells instead
+    // (mg_bottom_strips).  Of 1024, 4096, 16384: 2048^2 solve 3.88, 3.94, 4.40 ms (64^2 is quicker as a launch
+    // of its own), a served mix of 24 requests with levels of 45^2 to 55^2 261, 257, 278 ms.
+    long long bstrip_max = 3072;
+    std::vector<int> bstrip_host;
+    int* dbstrip = nullptr;
+    int nbstrip = 0;
     long long bottom_cells = 0;  // largest cell total of a problem's bottom levels (shared memory of mg_bottom)
     std::vector<long long> bottom_cells_host;  // per entry of bottom_host
     std::vector<KrylovDev> kd_host;
