@@ -11,7 +11,7 @@
 //   3. Everything else runs in a generic interpreter kernel over a postfix program expanded from the
 //      tree, again in the reference's operation order.
 #include "internal.h"
-#include "stencil.h"
+#include "stencil_exact.h"
 #include "pointwise.h"
 
 #include <algorithm>
@@ -483,47 +483,37 @@ __device__ __forceinline__ double div_h(double x, double h, double y, int p2) {
     return __fma_rn(r, y, q);
 }
 
-// one cell (box-relative index t) of the exact FTCS update, D terms (D <= 3; a compile-time D unrolls)
-__device__ __forceinline__ void ftcs_cell(const FieldView& in, const FieldView& out, const Box& box, const FtcsParams& P, long long t, int D) {
+// one cell (box-relative index t) of the exact update on a 1D mesh (2D and 3D: stencil_exact.h)
+__device__ __forceinline__ void ftcs_cell(const FieldView& in, const FieldView& out, const Box& box, const FtcsParams& P, long long t) {
     int i, j, k;
     box_index(t, box, i, j, k);
-    const long long o = (i - in.off[0]) + (j - in.off[1]) * in.sy + (k - in.off[2]) * in.sz;
-    const double c = in.data[o];
-    double sum = 0.;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        if (q >= D) break;
-        const int d = P.dims_order[q];
-        const long long st = d == 0 ? 1 : (d == 1 ? in.sy : in.sz);
-        const double l = in.data[o - st], r = in.data[o + st];
-        const double h = P.h[d], y = P.inv_h[d];
-        const int p2 = P.pow2[d];
-        const double a = div_h(__dsub_rn(r, c), h, y, p2);
-        const double b = div_h(__dsub_rn(c, l), h, y, p2);
-        const double d2 = div_h(__dsub_rn(a, b), h, y, p2);
-        sum = q == 0 ? d2 : __dadd_rn(sum, d2);
-    }
-    const long long oo = (i - out.off[0]) + (j - out.off[1]) * out.sy + (k - out.off[2]) * out.sz;
-    out.data[oo] = __dadd_rn(c, __dmul_rn(P.s, sum));
+    const long long o = i - in.off[0];
+    const double c = in.data[o], l = in.data[o - 1], r = in.data[o + 1];
+    const double h = P.h[0], y = P.inv_h[0];
+    const int p2 = P.pow2[0];
+    const double a = div_h(__dsub_rn(r, c), h, y, p2);
+    const double b = div_h(__dsub_rn(c, l), h, y, p2);
+    const double d2 = div_h(__dsub_rn(a, b), h, y, p2);
+    out.data[i - out.off[0]] = __dadd_rn(c, __dmul_rn(P.s, d2));
 }
 
-template <int D>
 __global__ void __launch_bounds__(256) ftcs_exact_kernel(FieldView in, FieldView out, Box box, FtcsParams P) {
-    const long long nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1], nz = box.hi[2] - box.lo[2];
-    const long long total = nx * ny * nz;
+    const long long total = box.count();
     for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x)
-        ftcs_cell(in, out, box, P, t, D);
+        ftcs_cell(in, out, box, P, t);
 }
 
 // Many assignments in one launch (opflow_assign_batch): a persistent grid takes tiles of every
 // assignment's box from one work queue (an atomic counter over the tile table), so grids of uneven
-// sizes and expressions of uneven cost share the launch.  An FTCS-shaped item takes the exact FTCS
-// cell (the values of the specialised kernels), any other the interpreter.
+// sizes and expressions of uneven cost share the launch.  FTCS-shaped 2D and 3D items take the exact
+// update's strips, a warp per tile, in a launch of their own (exact_batch_kernel).
 struct BatchItem {
     const Instr* prog;
     int nprog, arith;
-    int ftcs;          // 1: the exact FTCS update of `src`
+    int ftcs;          // 1: the exact FTCS update of `src` (1D: fp, else ax)
     FtcsParams fp;
+    AxisParams ax;
+    int mode;          // exact_mode(ax)
     FieldView src;
     LeafViews leaves;
     MeshPtrs mesh;
@@ -549,12 +539,21 @@ __global__ void __launch_bounds__(128) interp_batch_kernel(const BatchItem* __re
         const BatchTile T = tiles[c];
         const BatchItem& I = items[T.item];
         if (I.ftcs) {
-            for (long long t = T.t0 + threadIdx.x; t < T.t0 + T.n; t += blockDim.x) ftcs_cell(I.src, I.out, I.box, I.fp, t, I.fp.ndim);
+            for (long long t = T.t0 + threadIdx.x; t < T.t0 + T.n; t += blockDim.x) ftcs_cell(I.src, I.out, I.box, I.fp, t);
         } else {
             for (long long t = T.t0 + threadIdx.x; t < T.t0 + T.n; t += blockDim.x)
                 interp_cell(I.prog, I.nprog, I.leaves, I.mesh, I.box, I.out, I.cur, I.arith, t);
         }
     }
+}
+
+template <int ND>
+__global__ void __launch_bounds__(32 * EX_WARPS) exact_batch_kernel(const BatchItem* __restrict__ items, const ExactTile* __restrict__ tiles, int ntiles) {
+    const int t = blockIdx.x * EX_WARPS + (threadIdx.x >> 5);
+    if (t >= ntiles) return;  // (a whole warp)
+    const ExactTile T = tiles[t];
+    const BatchItem& I = items[T.item];
+    exact_dispatch(I.mode, [&](auto pm) { exact_tile<decltype(pm)::value, ND>(I.src, I.out, I.box, I.ax, T); });
 }
 
 // Markstein self-check: compares the three-operation quotient with __ddiv_rn on seeded operands that
@@ -1039,23 +1038,20 @@ static int build_plan(opflow_ctx ctx, opflow_field dst, int arith, const opflow_
                         OPG_TRY(markstein_ok(ctx, P.h[d], &good));
                         ok = ok && good;
                     }
+                AxisParams& A = plan->axis;
+                if (P.ndim >= 2) {
+                    std::memset(&A, 0, sizeof A);
+                    A.ndim = P.ndim;
+                    for (int d = 0; d < 3; ++d) {
+                        ok = axis_divisor(&A, d, P.h[d]) && ok;
+                        A.order[d] = d < P.ndim ? P.dims_order[d] : 0;
+                    }
+                    A.s = P.s;
+                }
                 if (ok) {
-                    plan->kind = PLAN_FTCS_EXACT;
+                    plan->kind = P.ndim >= 2 ? PLAN_AXIS_EXACT : PLAN_FTCS_EXACT;
                     plan->ftcs = P;
                     plan->src_slot = slot;
-                    if (P.ndim >= 2) {
-                        AxisParams& A = plan->axis;
-                        std::memset(&A, 0, sizeof A);
-                        A.ndim = P.ndim;
-                        for (int d = 0; d < 3; ++d) {
-                            A.h[d] = P.h[d];
-                            A.inv_h[d] = P.inv_h[d];
-                            A.pow2[d] = P.pow2[d];
-                            A.order[d] = d < P.ndim ? P.dims_order[d] : 0;
-                        }
-                        A.s = P.s;
-                        plan->kind = PLAN_AXIS_EXACT;
-                    }
                 }
             }
         }
@@ -1194,9 +1190,7 @@ static int run_plan(opflow_ctx ctx, opflow_field dst, int arith, const opflow_fi
             case PLAN_FTCS_EXACT: {
                 const FieldView in = leaves[plan->src_slot]->view();
                 const int g = grid_for(ctx, total, 256);
-                if (plan->ftcs.ndim == 1) ftcs_exact_kernel<1><<<g, 256, 0, ctx->stream>>>(in, out, plan->box, plan->ftcs);
-                else if (plan->ftcs.ndim == 2) ftcs_exact_kernel<2><<<g, 256, 0, ctx->stream>>>(in, out, plan->box, plan->ftcs);
-                else ftcs_exact_kernel<3><<<g, 256, 0, ctx->stream>>>(in, out, plan->box, plan->ftcs);
+                ftcs_exact_kernel<<<g, 256, 0, ctx->stream>>>(in, out, plan->box, plan->ftcs);
                 OPG_LAUNCHED();
                 OPG_TRY(check_launch("ftcs_exact_kernel"));
                 break;
@@ -1302,11 +1296,30 @@ int opflow_assign_batch(opflow_ctx ctx, int n, const opflow_field* dsts, const i
     if (rc) return rc;
     // tiles of every box; items for even and odd steps (aliased destinations swap buffers every step)
     std::vector<BatchTile> tiles;
+    std::vector<ExactTile> xtiles;  // the 2D items' first, then the 3D ones'
+    size_t xtiles2 = 0;
+    long long xcells = 0;
+    for (int i = 0; i < n; ++i)
+        if (plans[i].kind == PLAN_AXIS_EXACT) xcells += plans[i].box.count();
+    for (int D = 2; D <= 3; ++D) {
+        for (int i = 0; i < n; ++i) {
+            if (plans[i].kind != PLAN_AXIS_EXACT || plans[i].axis.ndim != D) continue;
+            // the items' tiles march as far as leaves the whole batch its share of tiles per SM
+            const Box& b = plans[i].box;
+            const long long total = b.count();
+            const int m = D - 1, march = exact_march(b, D, ctx->num_sms, (double) total / (double) std::max(1LL, xcells));
+            for (int a = b.lo[m]; total > 0 && a < b.hi[m]; a += march)
+                for (int y0 = b.lo[1]; y0 < (D == 3 ? b.hi[1] : b.lo[1] + 1); y0 += EX_ROWS)
+                    for (int x0 = b.lo[0]; x0 < b.hi[0]; x0 += EX_COLS) xtiles.push_back(ExactTile{i, x0, y0, a, std::min(a + march, b.hi[m])});
+        }
+        if (D == 2) xtiles2 = xtiles.size();
+    }
     for (int i = 0; i < n; ++i) {
+        if (plans[i].kind == PLAN_AXIS_EXACT) continue;
         const long long total = plans[i].box.count();
         for (long long t0 = 0; t0 < total; t0 += BATCH_TILE) tiles.push_back(BatchTile{i, (int) std::min<long long>(BATCH_TILE, total - t0), t0});
     }
-    if (tiles.size() > (size_t) 0x7fffffff) return fail(OPFLOW_E_INVALID, "too many tiles");
+    if (tiles.size() > (size_t) 0x7fffffff || xtiles.size() > (size_t) 0x7fffffff) return fail(OPFLOW_E_INVALID, "too many tiles");
     std::vector<BatchItem> items(2 * (size_t) n);
     for (int par = 0; par < 2; ++par)
         for (int i = 0; i < n; ++i) {
@@ -1324,28 +1337,44 @@ int opflow_assign_batch(opflow_ctx ctx, int n, const opflow_field* dsts, const i
             I.cur = front;
             I.ftcs = plans[i].kind == PLAN_FTCS_EXACT || plans[i].kind == PLAN_AXIS_EXACT;
             I.fp = plans[i].ftcs;
+            I.ax = plans[i].axis;
+            I.mode = exact_mode(plans[i].axis);
             if (I.ftcs) I.src = I.leaves.v[plans[i].src_slot];
         }
-    const size_t bytes_items = items.size() * sizeof(BatchItem), bytes_tiles = std::max<size_t>(1, tiles.size()) * sizeof(BatchTile);
-    const size_t bytes_prog = std::max<size_t>(1, progs.size()) * sizeof(Instr);
-    char* blob = (char*) dev_alloc(ctx, bytes_items + bytes_tiles + bytes_prog + 256);
-    if (!blob) return fail(OPFLOW_E_NOMEM, "batch tables");
     auto align = [](size_t v) { return (v + 15) & ~(size_t) 15; };
+    const size_t bytes_items = items.size() * sizeof(BatchItem), bytes_tiles = std::max<size_t>(1, tiles.size()) * sizeof(BatchTile);
+    const size_t bytes_prog = std::max<size_t>(1, progs.size()) * sizeof(Instr), bytes_x = std::max<size_t>(1, xtiles.size()) * sizeof(ExactTile);
+    char* blob = (char*) dev_alloc(ctx, align(bytes_items) + align(bytes_tiles) + align(bytes_prog) + align(bytes_x) + 256);
+    if (!blob) return fail(OPFLOW_E_NOMEM, "batch tables");
     BatchItem* d_items = (BatchItem*) blob;
     BatchTile* d_tiles = (BatchTile*) (blob + align(bytes_items));
     Instr* d_prog = (Instr*) (blob + align(bytes_items) + align(bytes_tiles));
-    int* d_next = (int*) (blob + align(bytes_items) + align(bytes_tiles) + align(bytes_prog));
+    ExactTile* d_xtiles = (ExactTile*) (blob + align(bytes_items) + align(bytes_tiles) + align(bytes_prog));
+    int* d_next = (int*) (blob + align(bytes_items) + align(bytes_tiles) + align(bytes_prog) + align(bytes_x));
     for (size_t q = 0; q < items.size(); ++q) items[q].prog = d_prog + prog_at[q % n];
     rc = OPFLOW_OK;
     if (cudaMemcpyAsync(d_items, items.data(), bytes_items, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
         (!tiles.empty() && cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(BatchTile), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) ||
+        (!xtiles.empty() && cudaMemcpyAsync(d_xtiles, xtiles.data(), xtiles.size() * sizeof(ExactTile), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) ||
         (!progs.empty() && cudaMemcpyAsync(d_prog, progs.data(), progs.size() * sizeof(Instr), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess))
         rc = fail(OPFLOW_E_CUDA, "batch tables upload failed");
     const int grid = (int) std::max<long long>(1, std::min<long long>((long long) tiles.size(), (long long) ctx->num_sms * 8));
     for (int s = 0; s < steps && rc == OPFLOW_OK; ++s) {
+        const BatchItem* step_items = d_items + (size_t) (s & 1) * n;
+        const int x2 = (int) xtiles2, x3 = (int) (xtiles.size() - xtiles2);
+        if (x2 > 0) {
+            exact_batch_kernel<2><<<(x2 + EX_WARPS - 1) / EX_WARPS, 32 * EX_WARPS, 0, ctx->stream>>>(step_items, d_xtiles, x2);
+            OPG_LAUNCHED();
+        }
+        if (x3 > 0) {
+            exact_batch_kernel<3><<<(x3 + EX_WARPS - 1) / EX_WARPS, 32 * EX_WARPS, 0, ctx->stream>>>(step_items, d_xtiles + x2, x3);
+            OPG_LAUNCHED();
+        }
+        rc = check_launch("exact_batch_kernel");
+        if (rc) break;
         if (!tiles.empty()) {
             if (cudaMemsetAsync(d_next, 0, sizeof(int), ctx->stream) != cudaSuccess) { rc = fail(OPFLOW_E_CUDA, "batch queue reset failed"); break; }
-            interp_batch_kernel<<<grid, 128, 0, ctx->stream>>>(d_items + (size_t) (s & 1) * n, d_tiles, (int) tiles.size(), d_next);
+            interp_batch_kernel<<<grid, 128, 0, ctx->stream>>>(step_items, d_tiles, (int) tiles.size(), d_next);
             OPG_LAUNCHED();
             rc = check_launch("interp_batch_kernel");
         }

@@ -14,10 +14,11 @@
 // A run of FAST steps on a Dirichlet node grid can keep the field in fixed point between its steps
 // (the resident kernels below): in 3D its steady-state steps stream their planes into shared memory
 // by TMA (axis3d_fxtma_kernel), in 2D a warp updates 30 columns x 8 rows with every load in flight.
-#include "stencil.h"
+#include "stencil_exact.h"
 #include "tma.h"
 #include "tune.h"
 
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -212,10 +213,9 @@ __global__ void __launch_bounds__(TX * TY) axis3d_kernel(FieldView in, FieldView
 // ------------------------------------------------------------------------------------------------ 2D
 constexpr int TX2 = 128;
 
-template <bool FAST>
 __global__ void __launch_bounds__(TX2) axis2d_kernel(FieldView in, FieldView out, Box box, AxisParams P, unsigned long long* maxslots, int step,
                                                      int ychunk) {
-    using T = typename std::conditional<FAST, long long, double>::type;
+    using T = long long;
     __shared__ T row[TX2 + 2];
     const int tx = threadIdx.x;
     const int x0 = box.lo[0] + blockIdx.x * TX2;
@@ -225,15 +225,9 @@ __global__ void __launch_bounds__(TX2) axis2d_kernel(FieldView in, FieldView out
     const int ys = box.lo[1] + blockIdx.y * ychunk;
     const int ye = min(ys + ychunk, box.hi[1]);
     if (ys >= ye) return;
-    int E = 0;
-    if (FAST) {
-        E = scale_exp(maxslots, step, P.bound_bits);
-        if (blockIdx.x == 0 && blockIdx.y == 0 && tx == 0) maxslots[(step + 2) % 3] = 0ull;
-    }
-    auto conv = [&](double v) -> T {
-        if constexpr (FAST) return fx_from(v, E);
-        else return v;
-    };
+    const int E = scale_exp(maxslots, step, P.bound_bits);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && tx == 0) maxslots[(step + 2) % 3] = 0ull;
+    auto conv = [&](double v) -> T { return fx_from(v, E); };
     const int k = box.lo[2];
     T below = conv(ld3(in, ic, ys - 1, k));
     T cur = conv(ld3(in, ic, ys, k));
@@ -246,32 +240,23 @@ __global__ void __launch_bounds__(TX2) axis2d_kernel(FieldView in, FieldView out
         __syncthreads();
         if (vx) {
             const T l = row[tx], r = row[tx + 2];
-            double v;
-            if constexpr (FAST) {
-                long long q = cur;
-                if (P.iso) {
-                    q += fx_mul((l - cur) + (r - cur) + (below - cur) + (above - cur), P.wm[0], P.wshift[0], P.wneg[0]);
-                } else {
-                    q += fx_mul((l - cur) + (r - cur), P.wm[0], P.wshift[0], P.wneg[0]);
-                    q += fx_mul((below - cur) + (above - cur), P.wm[1], P.wshift[1], P.wneg[1]);
-                }
-                v = fx_to(q, E);
-                const unsigned long long ab = (unsigned long long) __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
-                vmax = ab > vmax ? ab : vmax;
+            long long q = cur;
+            if (P.iso) {
+                q += fx_mul((l - cur) + (r - cur) + (below - cur) + (above - cur), P.wm[0], P.wshift[0], P.wneg[0]);
             } else {
-                double d2v[2];
-                d2v[0] = d2_exact(l, cur, r, P.h[0], P.inv_h[0], P.pow2[0]);
-                d2v[1] = d2_exact(below, cur, above, P.h[1], P.inv_h[1], P.pow2[1]);
-                double sum = __dadd_rn(d2v[P.order[0]], d2v[P.order[1]]);
-                v = __dadd_rn(cur, __dmul_rn(P.s, sum));
+                q += fx_mul((l - cur) + (r - cur), P.wm[0], P.wshift[0], P.wneg[0]);
+                q += fx_mul((below - cur) + (above - cur), P.wm[1], P.wshift[1], P.wneg[1]);
             }
+            const double v = fx_to(q, E);
+            const unsigned long long ab = (unsigned long long) __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+            vmax = ab > vmax ? ab : vmax;
             out.data[(long long) (i - out.off[0]) + (long long) (j - out.off[1]) * out.sy + (long long) (k - out.off[2]) * out.sz] = v;
         }
         __syncthreads();
         below = cur;
         cur = above;
     }
-    if (FAST) block_max_commit(vmax, &maxslots[(step + 1) % 3]);
+    block_max_commit(vmax, &maxslots[(step + 1) % 3]);
 }
 
 // ------------------------------------------------------------------------- 3D, register-blocked
@@ -283,10 +268,9 @@ constexpr int RB = 8;
 constexpr int RB_WARPS = 4;
 constexpr int RB_COLS = 30;
 
-template <bool FAST>
 __global__ void __launch_bounds__(32 * RB_WARPS, 4) axis3d_rb_kernel(FieldView in, FieldView out, Box box, AxisParams P, unsigned long long* maxslots,
                                                                   int step, int zchunk, int tiles_x, int tiles_y) {
-    using T = typename std::conditional<FAST, long long, double>::type;
+    using T = long long;
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * RB_WARPS + (threadIdx.x >> 5);
     if (warp >= tiles_x * tiles_y) return;
@@ -298,15 +282,9 @@ __global__ void __launch_bounds__(32 * RB_WARPS, 4) axis3d_rb_kernel(FieldView i
     const int zs = box.lo[2] + blockIdx.y * zchunk;
     const int ze = min(zs + zchunk, box.hi[2]);
     if (zs >= ze) return;
-    int E = 0;
-    if (FAST) {
-        E = scale_exp(maxslots, step, P.bound_bits);
-        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) maxslots[(step + 2) % 3] = 0ull;
-    }
-    auto conv = [&](double v) -> T {
-        if constexpr (FAST) return fx_from(v, E);
-        else return v;
-    };
+    const int E = scale_exp(maxslots, step, P.bound_bits);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) maxslots[(step + 2) % 3] = 0ull;
+    auto conv = [&](double v) -> T { return fx_from(v, E); };
     // row offsets of y0-1 .. y0+RB, clamped to the box edge + 1 (the farthest row the stencil reads)
     long long roff[RB + 2];
 #pragma unroll
@@ -341,30 +319,18 @@ __global__ void __launch_bounds__(32 * RB_WARPS, 4) axis3d_rb_kernel(FieldView i
             const int j = y0 + r;
             if (vx && j < box.hi[1]) {
                 const T b = cur[r], t = cur[r + 2], zb = below[r], za = above[r + 1];
-                double v;
-                if constexpr (FAST) {
-                    long long q = c;
-                    if (P.iso) {
-                        const long long z = (l - c) + (rr - c) + (b - c) + (t - c) + (zb - c) + (za - c);
-                        q += fx_mul(z, P.wm[0], P.wshift[0], P.wneg[0]);
-                    } else {
-                        q += fx_mul((l - c) + (rr - c), P.wm[0], P.wshift[0], P.wneg[0]);
-                        q += fx_mul((b - c) + (t - c), P.wm[1], P.wshift[1], P.wneg[1]);
-                        q += fx_mul((zb - c) + (za - c), P.wm[2], P.wshift[2], P.wneg[2]);
-                    }
-                    v = fx_to(q, E);
-                    const unsigned long long ab = (unsigned long long) __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
-                    vmax = ab > vmax ? ab : vmax;
+                long long q = c;
+                if (P.iso) {
+                    const long long z = (l - c) + (rr - c) + (b - c) + (t - c) + (zb - c) + (za - c);
+                    q += fx_mul(z, P.wm[0], P.wshift[0], P.wneg[0]);
                 } else {
-                    const double d0 = d2_exact(l, c, rr, P.h[0], P.inv_h[0], P.pow2[0]);
-                    const double d1 = d2_exact(b, c, t, P.h[1], P.inv_h[1], P.pow2[1]);
-                    const double d2 = d2_exact(zb, c, za, P.h[2], P.inv_h[2], P.pow2[2]);
-                    auto pick = [&](int a) { return a == 0 ? d0 : (a == 1 ? d1 : d2); };
-                    double sum = pick(P.order[0]);
-                    sum = __dadd_rn(sum, pick(P.order[1]));
-                    sum = __dadd_rn(sum, pick(P.order[2]));
-                    v = __dadd_rn(c, __dmul_rn(P.s, sum));
+                    q += fx_mul((l - c) + (rr - c), P.wm[0], P.wshift[0], P.wneg[0]);
+                    q += fx_mul((b - c) + (t - c), P.wm[1], P.wshift[1], P.wneg[1]);
+                    q += fx_mul((zb - c) + (za - c), P.wm[2], P.wshift[2], P.wneg[2]);
                 }
+                const double v = fx_to(q, E);
+                const unsigned long long ab = (unsigned long long) __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+                vmax = ab > vmax ? ab : vmax;
                 ocol[(long long) (j) * out.sy + (long long) k * out.sz] = v;
             }
         }
@@ -375,7 +341,7 @@ __global__ void __launch_bounds__(32 * RB_WARPS, 4) axis3d_rb_kernel(FieldView i
 #pragma unroll
         for (int r = 0; r < RB + 2; ++r) above[r] = conv(nxt[r]);
     }
-    if (FAST) block_max_commit(vmax, &maxslots[(step + 1) % 3]);
+    block_max_commit(vmax, &maxslots[(step + 1) % 3]);
 }
 
 // ------------------------------------------------------------- 3D, fixed point kept between steps
@@ -645,6 +611,96 @@ __global__ void __launch_bounds__(FT_THREADS, 4) axis3d_fxtma_kernel(const __gri
     }
 }
 
+// ------------------------------------------------------------------ exact update, a warp per tile
+template <int PM, int ND>
+__global__ void __launch_bounds__(32 * EX_WARPS) axis_exact_kernel(FieldView in, FieldView out, Box box, AxisParams P, int tiles_x, int tiles_y,
+                                                                 long long ntiles, int march) {
+    const long long t = (long long) blockIdx.x * EX_WARPS + (threadIdx.x >> 5);
+    if (t >= ntiles) return;  // (a whole warp)
+    const long long q = t / tiles_x;
+    ExactTile T;
+    T.item = 0;
+    T.x0 = box.lo[0] + (int) (t - q * tiles_x) * EX_COLS;
+    const int run = (int) (q / tiles_y), m = ND - 1;
+    T.y0 = box.lo[1] + (int) (q % tiles_y) * EX_ROWS;
+    T.a = box.lo[m] + run * march;
+    T.b = min(T.a + march, box.hi[m]);
+    exact_tile<PM, ND>(in, out, box, P, T);
+}
+
+static int launch_exact(opflow_ctx ctx, const FieldView& in, const FieldView& out, const Box& box, const AxisParams& P) {
+    const int nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1], m = P.ndim - 1;
+    const int tiles_x = (nx + EX_COLS - 1) / EX_COLS, tiles_y = P.ndim == 3 ? (ny + EX_ROWS - 1) / EX_ROWS : 1;
+    const int march = exact_march(box, P.ndim, ctx->num_sms, 1.0);
+    const long long n = (long long) tiles_x * tiles_y * ((box.hi[m] - box.lo[m] + march - 1) / march);
+    const long long g = (n + EX_WARPS - 1) / EX_WARPS;
+    if (g > 0x7fffffffLL) return fail(OPFLOW_E_UNSUPPORTED, "a box of %lld tiles", n);
+    exact_dispatch(exact_mode(P), [&](auto pm) {
+        constexpr int PM = decltype(pm)::value;
+        if (P.ndim == 2) axis_exact_kernel<(PM & 3), 2><<<(int) g, 32 * EX_WARPS, 0, ctx->stream>>>(in, out, box, P, tiles_x, tiles_y, n, march);
+        else axis_exact_kernel<PM, 3><<<(int) g, 32 * EX_WARPS, 0, ctx->stream>>>(in, out, box, P, tiles_x, tiles_y, n, march);
+    });
+    OPG_LAUNCHED();
+    return check_launch("axis_exact_kernel");
+}
+
+// How many significands x, and one of them, there are for which fma(x, ch, x * cl) with ch = RN(1/h),
+// cl = RN(1/h - ch) is not the correctly rounded x / h (no underflow).  (Correctly rounded multiplication
+// by a constant of which two words are kept: Brisebarre and Muller, IEEE Trans. Computers 57 (2008); the
+// search for the arguments that fail is done here for a reciprocal.)  cl is at most 2^-53 of 1/h, so
+// ch + cl is off 1/h by less than 2^-106 of it and the rounding of x cl is as small: the value before the
+// final rounding is off x / h by less than 2^-105 of it.  With the 53-bit significands X and H of x and h
+// the quotient is X / H and a rounding boundary is M / 2^E, M odd in [2^53, 2^54), E = 53 (X >= H) or 54:
+// the two can be confused only where |X 2^E - M H| < 4.  Each such X solves M H = -j (mod 2^E) for a small
+// j; those up to 8 are tried.  (Of 400000 h 1.2 % have one failing significand, none has two.)
+static int div2_failures(double h, unsigned long long* bad) {
+    const double ch = 1.0 / h, cl = std::fma(-ch, h, 1.0) / h;
+    int e, fails = 0;
+    const double m = std::frexp(h, &e);
+    const unsigned long long H = (unsigned long long) std::ldexp(m, 53);
+    const int a = __builtin_ctzll(H);
+    if (a > 3) return 0;  // M H and X 2^E are multiples of 16: no j up to 8
+    const unsigned long long Ho = H >> a;
+    unsigned long long inv = Ho;  // 1 / Ho modulo 2^64 (Newton)
+    for (int q = 0; q < 6; ++q) inv *= 2 - Ho * inv;
+    for (int E = 53; E <= 54; ++E)
+        for (int j = -8; j <= 8; ++j) {
+            if (j == 0 || (j & ((1 << a) - 1))) continue;
+            const unsigned long long mod = 1ull << (E - a);
+            unsigned long long M = (0ull - (unsigned long long) (long long) (j >> a)) * inv & (mod - 1);
+            if (M < (1ull << 53)) M += ((1ull << 53) - M + mod - 1) / mod * mod;
+            for (; M < (1ull << 54); M += mod) {
+                if (!(M & 1)) continue;
+                const unsigned long long X = (unsigned long long) (((unsigned __int128) M * H + (__int128) j) >> E);
+                if (X < (1ull << 52) || X >= (1ull << 53)) continue;
+                const double x = (double) X;
+                if (std::fma(x, ch, x * cl) != x / h) {
+                    ++fails;
+                    *bad = X;
+                }
+            }
+        }
+    return fails;
+}
+
+bool axis_divisor(AxisParams* P, int d, double h) {
+    int e;
+    P->h[d] = h;
+    P->inv_h[d] = 1.0 / h;
+    P->pow2[d] = std::frexp(h, &e) == 0.5;
+    P->shift[d] = 1 - e;  // h = 2^(e - 1)
+    P->cl[d] = std::fma(-P->inv_h[d], h, 1.0) / h;
+    P->guard[d] = 0;
+    if (!(h > 0) || e < -400 || e > 400) return false;
+    if (P->pow2[d]) return true;
+    unsigned long long bad = 0;
+    const int fails = div2_failures(h, &bad);
+    P->guard[d] = fails == 1;
+    P->bad_hi[d] = (int) (bad >> 32) & 0xFFFFF;
+    P->bad_lo[d] = (int) (unsigned) bad;
+    return fails <= 1;
+}
+
 // The TMA-staged steady-state step (default) or the register-blocked one: OPFLOW_FXRES_TMA=0|1, read at
 // every launch.
 static bool fxtma_enabled() {
@@ -759,9 +815,8 @@ int axis_launch_resident(opflow_ctx ctx, const FieldView& in, const FieldView& o
     return check_launch("axis3d_fxres_kernel");
 }
 
-// 3D tiling: register-blocked warps (the measured default for the fixed-point mode: integer-issue
-// bound, gains from the absent barriers) or shared-memory tiles (the default for the exact mode:
-// float64-pipe bound).  Both give the same values; the tuner times the two on the first launch of a
+// 3D tiling: warps that march their tile in registers (the default; fixed point: axis3d_rb_kernel, exact:
+// axis_exact_kernel) or shared-memory tiles (axis3d_kernel).  Both give the same values; the tuner times the two on the first launch of a
 // (mode, box, stencil) key (a repeated launch rewrites `out` and the max slot with the same values),
 // and OPFLOW_AXIS_TILING=register|smem overrides it, read at every launch.
 static int axis_launch_tiling(opflow_ctx ctx, const FieldView& in, const FieldView& out, const Box& box, const AxisParams& P, bool fast,
@@ -772,7 +827,7 @@ static bool use_register_tiles(opflow_ctx ctx, const FieldView& in, const FieldV
     const char* e = getenv("OPFLOW_AXIS_TILING");
     if (e && strcmp(e, "smem") == 0) return false;
     if (e && strcmp(e, "register") == 0) return true;
-    if (!tune_enabled()) return fast;
+    if (!tune_enabled()) return true;
     unsigned long long h = tune_hash(&P.ndim, sizeof P.ndim);
     h = tune_hash(P.h, sizeof P.h, h);
     h = tune_hash(P.inv_h, sizeof P.inv_h, h);
@@ -787,7 +842,7 @@ static bool use_register_tiles(opflow_ctx ctx, const FieldView& in, const FieldV
     char key[160];
     std::snprintf(key, sizeof key, "axis3d/%s/%dx%dx%d/%016llx", fast ? "fixed" : "exact", box.hi[0] - box.lo[0], box.hi[1] - box.lo[1],
                   box.hi[2] - box.lo[2], h);
-    const std::vector<int> cands = fast ? std::vector<int>{1, 0} : std::vector<int>{0, 1};
+    const std::vector<int> cands = {1, 0};
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return tune_cached(key, cands) == 1;
     return tune_pick(key, cands, [&](int reg) {
@@ -815,6 +870,7 @@ int axis_launch(opflow_ctx ctx, const FieldView& in, const FieldView& out, const
 static int axis_launch_tiling(opflow_ctx ctx, const FieldView& in, const FieldView& out, const Box& box, const AxisParams& P, bool fast,
                               unsigned long long* maxslots, int step, bool reg) {
     const int nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1], nz = box.hi[2] - box.lo[2];
+    if (!fast && (P.ndim == 2 || reg)) return launch_exact(ctx, in, out, box, P);
     if (P.ndim == 3 && reg) {
         const int tiles_x = (nx + RB_COLS - 1) / RB_COLS, tiles_y = (ny + RB - 1) / RB;
         const int bx = (tiles_x * tiles_y + RB_WARPS - 1) / RB_WARPS;
@@ -823,8 +879,7 @@ static int axis_launch_tiling(opflow_ctx ctx, const FieldView& in, const FieldVi
         const int zchunk = (nz + zchunks - 1) / zchunks;
         zchunks = (nz + zchunk - 1) / zchunk;
         dim3 g(bx, zchunks), b(32 * RB_WARPS);
-        if (fast) axis3d_rb_kernel<true><<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, zchunk, tiles_x, tiles_y);
-        else axis3d_rb_kernel<false><<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, zchunk, tiles_x, tiles_y);
+        axis3d_rb_kernel<<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, zchunk, tiles_x, tiles_y);
         OPG_LAUNCHED();
         return check_launch("axis3d_rb_kernel");
     }
@@ -848,8 +903,7 @@ static int axis_launch_tiling(opflow_ctx ctx, const FieldView& in, const FieldVi
         const int ychunk = (ny + ychunks - 1) / ychunks;
         ychunks = (ny + ychunk - 1) / ychunk;
         dim3 g(bx, ychunks), b(TX2);
-        if (fast) axis2d_kernel<true><<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, ychunk);
-        else axis2d_kernel<false><<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, ychunk);
+        axis2d_kernel<<<g, b, 0, ctx->stream>>>(in, out, box, P, maxslots, step, ychunk);
         OPG_LAUNCHED();
         return check_launch("axis2d_kernel");
     }

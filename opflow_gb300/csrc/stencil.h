@@ -10,7 +10,11 @@ struct AxisParams {
     int ndim;
     // EXACT: u + s * (d2<order[0]> + d2<order[1]> [+ d2<order[2]>]) with spacing h per dim
     double h[3], inv_h[3];
-    int pow2[3];
+    int pow2[3];                 // h is a power of two: division moves the exponent by shift
+    int shift[3];
+    double cl[3];                // RN(1/h - inv_h): x / h is fma(x, inv_h, x * cl) ...
+    int guard[3];                // ... except, where guard is set, for the x with this 52-bit fraction
+    int bad_hi[3], bad_lo[3];
     int order[3];
     double s;
     // FAST: u + sum_d w_d * ((u(i-e_d) - u) + (u(i+e_d) - u)) in fixed point
@@ -22,6 +26,8 @@ struct AxisParams {
 
 int axis_launch(opflow_ctx ctx, const FieldView& in, const FieldView& out, const Box& box, const AxisParams& P, bool fast,
                 unsigned long long* maxslots, int step);
+// Fills the divisor fields of dim d; false where this division by h is not available.
+bool axis_divisor(AxisParams* P, int d, double h);
 // One step of a run of fixed-point steps that keeps the update box in fixed point between steps (2D or
 // 3D; in 3D the steady-state steps stage their planes by TMA where the buffer's strides allow):
 // `first` reads float64, `last` writes float64; maxslots[0] holds the initial max|u| bit pattern.
