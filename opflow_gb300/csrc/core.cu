@@ -213,6 +213,40 @@ __device__ __forceinline__ double intp_exact(double x1, double y1, double x2, do
     return __ddiv_rn(__dsub_rn(__dmul_rn(a, y2), __dmul_rn(b, y1)), __dsub_rn(a, b));
 }
 
+// The value op (a mirror) gives the ghost cell at idx from its mirrored cell's value vm: xi, xm are the
+// cells' indices along op.dim.
+__device__ __forceinline__ double mirror_value(const PadOp& op, int ii, int im, double vm, const double* __restrict__ mx, const double* __restrict__ mdx) {
+    const double xi = mx[ii - op.es], xm = mx[im - op.es];
+    switch (op.bct) {
+        case OPFLOW_BC_DIRC:
+            if (op.corner) {
+                const double xb = mx[(op.side == 0 ? op.lstart : op.lend - 1) - op.es];
+                return intp_exact(xb, op.bcv, xm, vm, xi);
+            } else {
+                const double xb = mx[(op.side == 0 ? op.lstart : op.lend) - op.es];
+                return intp_exact(xb, op.bcv, __dadd_rn(xm, __ddiv_rn(mdx[im - op.es], 2.)), vm, __dadd_rn(xi, __ddiv_rn(mdx[ii - op.es], 2.)));
+            }
+        case OPFLOW_BC_NEUM:
+            if (op.corner) return __dadd_rn(vm, __dmul_rn(op.bcv, __dsub_rn(xi, xm)));
+            else {
+                // x(idx) + dx(idx)/2 - x(mirror) - dx(mirror)/2, left to right
+                double t = __dadd_rn(xi, __ddiv_rn(mdx[ii - op.es], 2.));
+                t = __dsub_rn(t, xm);
+                t = __dsub_rn(t, __ddiv_rn(mdx[im - op.es], 2.));
+                return __dadd_rn(vm, __dmul_rn(op.bcv, t));
+            }
+        case OPFLOW_BC_ASYMM: return -vm;
+        default: return vm;  // SYMM
+    }
+}
+
+// the cell along op.dim that op reads for index i
+__device__ __forceinline__ int pad_source(const PadOp& op, int i) {
+    if (op.kind == PAD_PERIODIC) return i + (op.side == 0 ? op.period : -op.period);
+    if (op.corner) return op.side == 0 ? 2 * op.lstart - i : 2 * op.lend - 2 - i;
+    return op.side == 0 ? 2 * op.lstart - 1 - i : 2 * op.lend - 1 - i;
+}
+
 __global__ void pad_kernel(FieldView f, PadOp op, const double* __restrict__ mx, const double* __restrict__ mdx) {
     const long long nx = op.hi[0] - op.lo[0], ny = op.hi[1] - op.lo[1], nz = op.hi[2] - op.lo[2];
     const long long total = nx * ny * nz;
@@ -227,46 +261,81 @@ __global__ void pad_kernel(FieldView f, PadOp op, const double* __restrict__ mx,
             continue;
         }
         int mi[3] = {idx[0], idx[1], idx[2]};
-        const int i = op.dim;
-        if (op.kind == PAD_PERIODIC) {
-            mi[i] += op.side == 0 ? op.period : -op.period;
-        } else if (op.corner) {
-            mi[i] = op.side == 0 ? 2 * op.lstart - idx[i] : 2 * op.lend - 2 - idx[i];
-        } else {
-            mi[i] = op.side == 0 ? 2 * op.lstart - 1 - idx[i] : 2 * op.lend - 1 - idx[i];
-        }
-        const long long om = (mi[0] - f.off[0]) + (mi[1] - f.off[1]) * f.sy + (mi[2] - f.off[2]) * f.sz;
-        const double vm = f.data[om];
-        double v = vm;
-        if (op.kind == PAD_MIRROR) {
-            const double xi = mx[idx[i] - op.es], xm = mx[mi[i] - op.es];
-            switch (op.bct) {
-                case OPFLOW_BC_DIRC:
-                    if (op.corner) {
-                        const double xb = mx[(op.side == 0 ? op.lstart : op.lend - 1) - op.es];
-                        v = intp_exact(xb, op.bcv, xm, vm, xi);
-                    } else {
-                        const double xb = mx[(op.side == 0 ? op.lstart : op.lend) - op.es];
-                        v = intp_exact(xb, op.bcv, __dadd_rn(xm, __ddiv_rn(mdx[mi[i] - op.es], 2.)), vm,
-                                       __dadd_rn(xi, __ddiv_rn(mdx[idx[i] - op.es], 2.)));
-                    }
-                    break;
-                case OPFLOW_BC_NEUM:
-                    if (op.corner) v = __dadd_rn(vm, __dmul_rn(op.bcv, __dsub_rn(xi, xm)));
-                    else {
-                        // x(idx) + dx(idx)/2 - x(mirror) - dx(mirror)/2, left to right
-                        double t = __dadd_rn(xi, __ddiv_rn(mdx[idx[i] - op.es], 2.));
-                        t = __dsub_rn(t, xm);
-                        t = __dsub_rn(t, __ddiv_rn(mdx[mi[i] - op.es], 2.));
-                        v = __dadd_rn(vm, __dmul_rn(op.bcv, t));
-                    }
-                    break;
-                case OPFLOW_BC_SYMM: v = vm; break;
-                case OPFLOW_BC_ASYMM: v = -vm; break;
-            }
-        }
-        f.data[o] = v;
+        mi[op.dim] = pad_source(op, idx[op.dim]);
+        const double vm = f.data[(mi[0] - f.off[0]) + (mi[1] - f.off[1]) * f.sy + (mi[2] - f.off[2]) * f.sz];
+        f.data[o] = op.kind == PAD_MIRROR ? mirror_value(op, idx[op.dim], mi[op.dim], vm, mx, mdx) : vm;
     }
+}
+
+// ---- a field's whole padding update in one launch ----------------------------------------------------
+// The zones of updatePadding are filled one after another, later ones reading what earlier ones wrote.
+// Instead every ghost cell is computed on its own: the last zone that holds it says which cell it is made
+// from, that cell is again looked for in the zones before it, down to a cell that no zone writes (or a
+// fill), and the zones' operations are applied on the way back.  A zone reads along its own dim inside
+// the range and along the others only what earlier zones wrote, so the chain ends in a cell that this
+// launch does not write, and the values are those of the zones in turn.  (A periodic zone wider than its
+// period reads itself: such fields keep the zones in turn.)  The update of a small field is all launch
+// latency: 64 fields' Dirichlet nodes took 256 launches, 0.6 ms.
+constexpr int PAD_MAX = 12;  // corner Dirichlet fills (at most 6), then mirror or periodic zones (at most 6)
+struct PadList {
+    int n = 0;
+    PadOp op[PAD_MAX];
+    long long start[PAD_MAX + 1];  // first cell of each zone in the launch's numbering
+};
+struct PadJob {
+    FieldView f;
+    const double *x[3], *dx[3];
+    PadList L;
+};
+
+__device__ __forceinline__ void pad_cell(const PadJob& J, long long t) {
+    int z = 0;
+    while (t >= J.L.start[z + 1]) ++z;
+    Box bx;
+    for (int d = 0; d < 3; ++d) { bx.lo[d] = J.L.op[z].lo[d]; bx.hi[d] = J.L.op[z].hi[d]; }
+    int idx[3];
+    box_index(t - J.L.start[z], bx, idx[0], idx[1], idx[2]);
+    const FieldView& f = J.f;
+    const long long o = (idx[0] - f.off[0]) + (idx[1] - f.off[1]) * f.sy + (idx[2] - f.off[2]) * f.sz;
+    // the chain of zones, last writer first: at most one mirror or periodic zone per dim, then a fill
+    int chain[4], from[4], depth = 0, limit = J.L.n;
+    double v = 0.;
+    bool filled = false;
+    for (; depth < 4;) {
+        int q = limit - 1;
+        for (; q >= 0; --q) {
+            const PadOp& p = J.L.op[q];
+            if (idx[0] >= p.lo[0] && idx[0] < p.hi[0] && idx[1] >= p.lo[1] && idx[1] < p.hi[1] && idx[2] >= p.lo[2] && idx[2] < p.hi[2]) break;
+        }
+        if (q < 0) break;
+        const PadOp& p = J.L.op[q];
+        if (p.kind == PAD_FILL) {
+            v = p.bcv;
+            filled = true;
+            break;
+        }
+        chain[depth] = q;
+        from[depth++] = idx[p.dim];
+        idx[p.dim] = pad_source(p, idx[p.dim]);
+        limit = q;
+    }
+    if (!filled) v = f.data[(idx[0] - f.off[0]) + (idx[1] - f.off[1]) * f.sy + (idx[2] - f.off[2]) * f.sz];
+    while (depth-- > 0) {
+        const PadOp& p = J.L.op[chain[depth]];
+        if (p.kind == PAD_MIRROR) v = mirror_value(p, from[depth], pad_source(p, from[depth]), v, J.x[p.dim], J.dx[p.dim]);
+    }
+    f.data[o] = v;
+}
+
+__global__ void __launch_bounds__(256) pad_field_kernel(const __grid_constant__ PadJob J) {
+    const long long total = J.L.start[J.L.n];
+    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x) pad_cell(J, t);
+}
+// block row y: job y
+__global__ void __launch_bounds__(256) pad_jobs_kernel(const PadJob* __restrict__ jobs) {
+    const PadJob& J = jobs[blockIdx.y];
+    const long long total = J.L.start[J.L.n];
+    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x) pad_cell(J, t);
 }
 
 static int launch_pad_box(opflow_field f, double* data, const PadOp& op) {
@@ -302,6 +371,7 @@ static int launch_pad(opflow_field f, double* data, const PadOp& op) {
 }
 
 int update_padding_full(opflow_field f, double* data);
+bool padding_self_overlaps(opflow_field f);
 
 // Step 0 (Dirichlet values on corner-located boundary nodes) is idempotent with what the kernels write,
 // step 1 mirrors, step 2 periodic copies, in the reference's order.
@@ -313,34 +383,16 @@ int update_padding_buf(opflow_field f, double* data) {
     return OPFLOW_OK;
 }
 
-// The corner-located Dirichlet boundary nodes of `data` (the writes updatePadding makes for a field
-// without a ghost layer, in its order) filled with values[d][side] instead of the boundary values: a
-// resident fixed-point run stores the boundary constants there as fixed-point bit patterns between its
-// steps, and update_padding_full puts the float64 constants back afterwards.
-int fill_dirichlet_nodes(opflow_field f, double* data, const double values[3][2]) {
-    const opflow_field_info& R = f->info;
-    const opflow_field_desc& F = f->desc;
-    for (int i = 0; i < R.ndim; ++i)
-        for (int side = 0; side < 2; ++side) {
-            const bool at = side == 0 ? R.local[i][0] == R.accessible[i][0] : R.local[i][1] == R.accessible[i][1];
-            if (at && F.bc_type[i][side] == OPFLOW_BC_DIRC && F.loc[i] == OPFLOW_CORNER) {
-                PadOp op{};
-                op.kind = PAD_FILL;
-                op.dim = i;
-                op.bcv = values[i][side];
-                for (int k = 0; k < 3; ++k) { op.lo[k] = R.local[k][0]; op.hi[k] = R.local[k][1]; }
-                op.lo[i] = side == 0 ? R.local[i][0] : R.local[i][1] - 1;
-                op.hi[i] = op.lo[i] + 1;
-                OPG_TRY(launch_pad(f, data, op));
-            }
-        }
-    return OPFLOW_OK;
-}
-
-int update_padding_full(opflow_field f, double* data) {
+// updatePadding's zones in their order, the empty ones left out
+static void pad_zones(opflow_field f, std::vector<PadOp>& zones) {
     const opflow_field_info& R = f->info;
     const opflow_field_desc& F = f->desc;
     const int D = R.ndim;
+    auto add = [&](const PadOp& op) {
+        Box b;
+        for (int d = 0; d < 3; ++d) { b.lo[d] = op.lo[d]; b.hi[d] = op.hi[d]; }
+        if (b.count() > 0) zones.push_back(op);
+    };
     for (int i = 0; i < D; ++i) {
         for (int side = 0; side < 2; ++side) {
             const bool at = side == 0 ? R.local[i][0] == R.accessible[i][0] : R.local[i][1] == R.accessible[i][1];
@@ -348,11 +400,12 @@ int update_padding_full(opflow_field f, double* data) {
                 PadOp op{};
                 op.kind = PAD_FILL;
                 op.dim = i;
+                op.side = side;
                 op.bcv = F.bc_value[i][side];
                 for (int k = 0; k < 3; ++k) { op.lo[k] = R.local[k][0]; op.hi[k] = R.local[k][1]; }
                 op.lo[i] = side == 0 ? R.local[i][0] : R.local[i][1] - 1;
                 op.hi[i] = op.lo[i] + 1;
-                OPG_TRY(launch_pad(f, data, op));
+                add(op);
             }
         }
     }
@@ -382,7 +435,7 @@ int update_padding_full(opflow_field f, double* data) {
             for (int j = 0; j < i; ++j) { op.lo[j] = st[j]; op.hi[j] = en[j]; }
             if (side == 0) { op.lo[i] = st[i]; op.hi[i] = R.local[i][0]; }
             else { op.lo[i] = R.local[i][1]; op.hi[i] = R.logical[i][1]; }
-            OPG_TRY(launch_pad(f, data, op));
+            add(op);
         }
     }
     for (int i = 0; i < D; ++i) {
@@ -396,10 +449,67 @@ int update_padding_full(opflow_field f, double* data) {
             for (int k = 0; k < 3; ++k) { op.lo[k] = R.logical[k][0]; op.hi[k] = R.logical[k][1]; }
             if (side == 0) { op.lo[i] = R.logical[i][0]; op.hi[i] = R.accessible[i][0]; }
             else { op.lo[i] = R.accessible[i][1]; op.hi[i] = R.logical[i][1]; }
-            OPG_TRY(launch_pad(f, data, op));
+            add(op);
         }
     }
-    return OPFLOW_OK;
+}
+
+// One launch's description of the whole update of `data`; false where the zones have to run in turn.
+static bool pad_job(opflow_field f, double* data, const std::vector<PadOp>& zones, PadJob* J) {
+    if (zones.size() > (size_t) PAD_MAX || padding_self_overlaps(f)) return false;
+    J->f = f->view();
+    J->f.data = data;
+    for (int d = 0; d < 3; ++d) {
+        J->x[d] = f->mesh->x[d];
+        J->dx[d] = f->mesh->dx[d];
+    }
+    PadList& L = J->L;
+    L.n = 0;
+    L.start[0] = 0;
+    for (const PadOp& op : zones) {
+        // (a mirror zone wider than the range reads the other side's zone, also a later one's old values)
+        if (op.kind == PAD_MIRROR && op.hi[op.dim] - op.lo[op.dim] > op.lend - op.lstart - (op.corner ? 1 : 0)) return false;
+        long long c = 1;
+        for (int d = 0; d < 3; ++d) c *= op.hi[d] - op.lo[d];
+        L.op[L.n] = op;
+        L.start[L.n + 1] = L.start[L.n] + c;
+        ++L.n;
+    }
+    return true;
+}
+
+static int run_zones(opflow_field f, double* data, const std::vector<PadOp>& zones) {
+    if (zones.empty()) return OPFLOW_OK;
+    PadJob J;
+    if (!pad_job(f, data, zones, &J)) {
+        for (const PadOp& op : zones) OPG_TRY(launch_pad(f, data, op));
+        return OPFLOW_OK;
+    }
+    const long long blocks = std::min<long long>((J.L.start[J.L.n] + 255) / 256, 4096);
+    pad_field_kernel<<<(int) blocks, 256, 0, f->ctx->stream>>>(J);
+    OPG_LAUNCHED();
+    return check_launch("pad_field_kernel");
+}
+
+int update_padding_full(opflow_field f, double* data) {
+    std::vector<PadOp> zones;
+    pad_zones(f, zones);
+    return run_zones(f, data, zones);
+}
+
+// The corner-located Dirichlet boundary nodes of `data` (the writes updatePadding makes for a field
+// without a ghost layer, in its order) filled with values[d][side] instead of the boundary values: a
+// resident fixed-point run stores the boundary constants there as fixed-point bit patterns between its
+// steps, and update_padding_full puts the float64 constants back afterwards.
+int fill_dirichlet_nodes(opflow_field f, double* data, const double values[3][2]) {
+    std::vector<PadOp> zones, fills;
+    pad_zones(f, zones);
+    for (PadOp& op : zones)
+        if (op.kind == PAD_FILL) {
+            op.bcv = values[op.dim][op.side];
+            fills.push_back(op);
+        }
+    return run_zones(f, data, fills);
 }
 
 bool padding_self_overlaps(opflow_field f) {
@@ -415,6 +525,44 @@ int update_padding_assign(opflow_field f) {
     OPG_TRY(update_padding_buf(f, f->buf[f->cur]));
     if (padding_self_overlaps(f)) OPG_TRY(update_padding_full(f, f->buf[f->cur]));
     return OPFLOW_OK;
+}
+
+int update_padding_assign_many(opflow_ctx ctx, const opflow_field* fs, int n) {
+    std::vector<PadJob> jobs;
+    long long most = 0;
+    for (int i = 0; i < n; ++i) {
+        opflow_field f = fs[i];
+        double* data = f->buf[f->cur];
+        if (f->padding_is_step0_only() && f->bc_fresh[f->cur]) continue;
+        std::vector<PadOp> zones;
+        pad_zones(f, zones);
+        PadJob J;
+        if (zones.empty()) {
+            f->bc_fresh[f->cur] = true;
+        } else if (pad_job(f, data, zones, &J)) {
+            jobs.push_back(J);
+            most = std::max(most, J.L.start[J.L.n]);
+            f->bc_fresh[f->cur] = true;
+        } else {
+            OPG_TRY(update_padding_assign(f));
+        }
+    }
+    if (jobs.empty()) return OPFLOW_OK;
+    PadJob* d = (PadJob*) dev_alloc(ctx, jobs.size() * sizeof(PadJob));
+    if (!d) return fail(OPFLOW_E_NOMEM, "padding table");
+    int rc = OPFLOW_OK;
+    // (the table is read by the copy before this returns: the stream is synchronised below)
+    if (cudaMemcpyAsync(d, jobs.data(), jobs.size() * sizeof(PadJob), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+        rc = fail(OPFLOW_E_CUDA, "padding table upload failed");
+    for (size_t at = 0; at < jobs.size() && rc == OPFLOW_OK; at += 32768) {
+        const dim3 g((unsigned) std::min<long long>((most + 255) / 256, 64), (unsigned) std::min<size_t>(jobs.size() - at, 32768));
+        pad_jobs_kernel<<<g, 256, 0, ctx->stream>>>(d + at);
+        OPG_LAUNCHED();
+        rc = check_launch("pad_jobs_kernel");
+    }
+    dev_free(ctx, d);
+    if (rc == OPFLOW_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = fail(OPFLOW_E_CUDA, "padding update failed: %s", cudaGetErrorString(cudaGetLastError()));
+    return rc;
 }
 
 int ensure_back(opflow_field f) {

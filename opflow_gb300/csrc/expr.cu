@@ -1378,11 +1378,11 @@ int opflow_assign_batch(opflow_ctx ctx, int n, const opflow_field* dsts, const i
             OPG_LAUNCHED();
             rc = check_launch("interp_batch_kernel");
         }
-        for (int i = 0; i < n && rc == OPFLOW_OK; ++i) {
+        for (int i = 0; i < n; ++i) {
             if (plans[i].aliased) dsts[i]->cur = 1 - dsts[i]->cur;
             dsts[i]->version++;
-            rc = update_padding_assign(dsts[i]);
         }
+        if (rc == OPFLOW_OK) rc = update_padding_assign_many(ctx, dsts, n);
     }
     dev_free(ctx, blob);
     if (rc == OPFLOW_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = fail(OPFLOW_E_CUDA, "batched assign failed: %s", cudaGetErrorString(cudaGetLastError()));

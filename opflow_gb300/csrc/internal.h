@@ -128,6 +128,9 @@ int fill_dirichlet_nodes(opflow_field f, double* data, const double values[3][2]
 // updatePadding as an assignment does it (assign_impl and assignImpl_final each run one pass; a second
 // pass only changes a periodic zone wider than its period)
 int update_padding_assign(opflow_field f);
+// the same for many fields of one context, their zones in one launch; synchronises the stream where
+// anything was to be done
+int update_padding_assign_many(opflow_ctx ctx, const opflow_field* fs, int n);
 bool padding_self_overlaps(opflow_field f);
 int ensure_scratch(opflow_ctx ctx, size_t bytes);
 // Device memory of a context: stream-ordered allocations on the context's stream from a per-device
