@@ -400,17 +400,19 @@ done_chain:
 // RHS_ONLY: the right-hand side alone (generateb): the same program on the pads' bias parts, which no
 // coefficient ever feeds, so b is bit-identical to the full assembly's
 template <bool RHS_ONLY>
-__global__ void __launch_bounds__(128) assemble_kernel(const PInstr* __restrict__ prog, int nprog, AsmParams P, double* __restrict__ coef,
-                                                       double* __restrict__ rhs, int* __restrict__ err) {
+__global__ void __launch_bounds__(128) assemble_kernel(const PInstr* __restrict__ prog, int nprog, AsmParams P, AsmCells cells,
+                                                       double* __restrict__ coef, double* __restrict__ rhs, int* __restrict__ err) {
     const int NK = RHS_ONLY ? 0 : P.nk;
     const long long nx = P.box.hi[0] - P.box.lo[0], ny = P.box.hi[1] - P.box.lo[1], nz = P.box.hi[2] - P.box.lo[2];
     const long long total = nx * ny * nz;
     // the last divisor of a pad / num step and its reciprocal RN(1 / num): on a uniform mesh the same
     // spacing divides every difference, so the float64 division runs once per thread, not per use
     double last_div = 0., last_rec = __ddiv_rn(1., 0.);
-    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x) {
-        int cell[3];
-        box_index(t, P.box, cell[0], cell[1], cell[2]);
+    for (long long q = blockIdx.x * (long long) blockDim.x + threadIdx.x; q < cells.start[cells.n]; q += (long long) gridDim.x * blockDim.x) {
+        int cell[3], z = 0;
+        while (q >= cells.start[z + 1]) ++z;
+        box_index(q - cells.start[z], cells.box[z], cell[0], cell[1], cell[2]);
+        const long long t = (cell[0] - P.box.lo[0]) + nx * ((cell[1] - P.box.lo[1]) + ny * (cell[2] - P.box.lo[2]));
         // two stacks: StencilPad values (operands that depend on the unknown) and plain numbers; every
         // instruction knows statically which of its operands are pads (ta, tb)
         PadVal st[PAD_STACK];
@@ -513,6 +515,72 @@ __global__ void __launch_bounds__(128) assemble_kernel(const PInstr* __restrict_
         }
         rhs[t] = -st[0].b;
     }
+}
+
+// the inner cells' right-hand side where it is plain (AsmPlan): b = -bias = sign x field; a block row per row
+// of cells (grid-stride)
+__global__ void __launch_bounds__(256) plain_rhs_kernel(FieldView f, Box box, Box inner, int o0, int o1, int o2, double sign, double* __restrict__ rhs) {
+    const int nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1];
+    const int jn = inner.hi[1] - inner.lo[1], rows = jn * (inner.hi[2] - inner.lo[2]);
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+        const int k = inner.lo[2] + r / jn, j = inner.lo[1] + r % jn;
+        const double* src = f.data + (o0 - f.off[0]) + (long long) (j + o1 - f.off[1]) * f.sy + (long long) (k + o2 - f.off[2]) * f.sz;
+        double* dst = rhs + (long long) nx * ((j - box.lo[1]) + (long long) ny * (k - box.lo[2])) - box.lo[0];
+        for (int i = inner.lo[0] + blockIdx.x * blockDim.x + threadIdx.x; i < inner.hi[0]; i += gridDim.x * blockDim.x)
+            dst[i] = sign == 0. ? 0. : __dmul_rn(sign, src[i]);
+    }
+}
+
+// What the bias program makes of zero leaves: the plain form of the inner cells' right-hand side, if it has
+// one.  Zero biases stay zero under sums and under products with finite constants (a field's value as a
+// factor could be infinite); 0 + f, f + (0 x -1) and 0 + (-f) are +-f.
+static void plain_rhs(const std::vector<PInstr>& prog, AsmPlan* plan) {
+    struct V { int kind; double v; PInstr in; };  // 0: zero bias / constant v, 1: v x the load `in`, 2: anything else
+    std::vector<V> pads, nums;
+    const V other{2, 0., PInstr{}};
+    for (const PInstr& in : prog) {
+        switch (in.op) {
+            case Q_LOADU: pads.push_back(V{0, 0., PInstr{}}); break;
+            case Q_LOADS: nums.push_back(V{1, 1., in}); break;
+            case Q_CONST: nums.push_back(std::isfinite(in.v) ? V{0, in.v, PInstr{}} : other); break;
+            case Q_DX: case Q_X: nums.push_back(other); break;
+            case Q_NEG: {
+                auto& st = in.ta ? pads : nums;
+                st.back().v = -st.back().v;
+                break;
+            }
+            case Q_NOT: case Q_F1: nums.back() = other; break;
+            case Q_SEL: nums.pop_back(); nums.pop_back(); nums.back() = other; break;
+            case Q_GT: case Q_GE: case Q_LT: case Q_LE: case Q_NE: case Q_AND: case Q_OR: case Q_F2: nums.pop_back(); nums.back() = other; break;
+            default: {
+                if (!in.ta && !in.tb) {
+                    nums.pop_back();
+                    nums.back() = other;
+                    break;
+                }
+                V b, a;
+                if (in.tb) { b = pads.back(); pads.pop_back(); } else { b = nums.back(); nums.pop_back(); }
+                if (in.ta) { a = pads.back(); pads.pop_back(); } else { a = nums.back(); nums.pop_back(); }
+                V r = other;
+                const bool za = in.ta && a.kind == 0 && a.v == 0., zb = in.tb && b.kind == 0 && b.v == 0.;
+                if (in.op == Q_ADD || in.op == Q_SUB) {
+                    if (za && zb) r = a;
+                    else if (za && b.kind == 1) { r = b; if (in.op == Q_SUB) r.v = -r.v; }
+                    else if (zb && a.kind == 1) r = a;
+                } else if (za && !in.tb && b.kind == 0 && (in.op == Q_MUL || (in.op == Q_DIV && b.v != 0. && std::isfinite(1. / b.v)))) {
+                    r = a;
+                } else if (zb && !in.ta && a.kind == 0 && in.op == Q_MUL) {
+                    r = b;
+                }
+                pads.push_back(r);
+            }
+        }
+    }
+    const V& r = pads.back();
+    plan->rhs_plain = (r.kind == 0 && r.v == 0.) || (r.kind == 1 && std::fabs(r.v) == 1.);
+    plan->rhs_sign = r.kind == 1 ? -r.v : 0.;  // rhs = -bias
+    plan->rhs_slot = r.in.slot;
+    for (int d = 0; d < 3; ++d) plan->rhs_off[d] = r.in.off[d];
 }
 
 // ======================================================================== host structural evaluation
@@ -682,6 +750,14 @@ int asm_prepare(opflow_ctx ctx, opflow_field target, const opflow_node* nodes, i
             if (lo < P.st_log[d][0] || hi >= P.st_log[d][1]) return fail(OPFLOW_E_RANGE, "unknown read outside its logical range along dim %d", d);
         }
     plan->prog = C.prog;
+    plain_rhs(C.prog, plan);
+    plan->inner = P.box;
+    for (auto& o : C.uoffs)
+        for (int d = 0; d < 3; ++d) {
+            if (d >= R.ndim) continue;
+            plan->inner.lo[d] = std::max(plan->inner.lo[d], P.st_asg[d][0] - o[d]);
+            plan->inner.hi[d] = std::min(plan->inner.hi[d], P.st_asg[d][1] - o[d]);
+        }
     // middle cell's key order (HYPREEqnSolveHandler.hpp:97-107)
     int mid[3] = {0, 0, 0};
     for (int d = 0; d < R.ndim; ++d) mid[d] = (R.assignable[d][0] + R.assignable[d][1]) / 2;
@@ -703,11 +779,41 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
     int* err = (int*) ctx->scratch;
     cudaMemsetAsync(err, 0, sizeof(int), ctx->stream);
     cudaMemcpyAsync(dprog, plan->prog.data(), plan->prog.size() * sizeof(PInstr), cudaMemcpyHostToDevice, ctx->stream);
-    long long blocks = (N + 127) / 128;
-    if (blocks > (long long) ctx->num_sms * 32) blocks = (long long) ctx->num_sms * 32;
-    if (coef) assemble_kernel<false><<<(int) blocks, 128, 0, ctx->stream>>>(dprog, (int) plan->prog.size(), plan->P, coef, rhs, err);
-    else assemble_kernel<true><<<(int) blocks, 128, 0, ctx->stream>>>(dprog, (int) plan->prog.size(), plan->P, coef, rhs, err);
-    OPG_LAUNCHED();
+    // the right-hand side alone: inner cells as one plain field where they are, the shell around them by
+    // the program (256^3 cells of f == d2x(p) + d2y(p) + d2z(p): 3.39 ms by the program, about 50 us here)
+    AsmCells cells;
+    auto add = [&](const Box& b) {
+        if (b.empty()) return;
+        cells.box[cells.n] = b;
+        cells.start[cells.n + 1] = cells.start[cells.n] + b.count();
+        ++cells.n;
+    };
+    cells.start[0] = 0;
+    const Box &all = plan->P.box, &in = plan->inner;
+    if (!coef && plan->rhs_plain && !plan->P.pin && !in.empty()) {
+        const int nx = in.hi[0] - in.lo[0], rows = (in.hi[1] - in.lo[1]) * (in.hi[2] - in.lo[2]);
+        plain_rhs_kernel<<<dim3((nx + 255) / 256, std::min(rows, 65535)), 256, 0, ctx->stream>>>(plan->P.leaves[plan->rhs_slot], all, in, plan->rhs_off[0],
+                                                                                            plan->rhs_off[1], plan->rhs_off[2], plan->rhs_sign, rhs);
+        OPG_LAUNCHED();
+        Box rest = all;
+        for (int d = 2; d >= 0; --d) {
+            Box lo = rest, hi = rest;
+            lo.hi[d] = in.lo[d];
+            hi.lo[d] = in.hi[d];
+            add(lo);
+            add(hi);
+            rest.lo[d] = in.lo[d];
+            rest.hi[d] = in.hi[d];
+        }
+    } else {
+        add(all);
+    }
+    const long long blocks = std::min((cells.start[cells.n] + 127) / 128, (long long) ctx->num_sms * 32);
+    if (blocks > 0) {
+        if (coef) assemble_kernel<false><<<(int) blocks, 128, 0, ctx->stream>>>(dprog, (int) plan->prog.size(), plan->P, cells, coef, rhs, err);
+        else assemble_kernel<true><<<(int) blocks, 128, 0, ctx->stream>>>(dprog, (int) plan->prog.size(), plan->P, cells, coef, rhs, err);
+        OPG_LAUNCHED();
+    }
     int rc = check_launch("assemble_kernel");
     int herr = 0;
     cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);

@@ -37,8 +37,22 @@ struct AsmParams {
     FieldView leaves[8];
 };
 
+// The cells of a kernel run: the boxes' cells, one box after another (start: first cell of each box).
+struct AsmCells {
+    int n = 0;
+    Box box[7];
+    long long start[8];
+};
+
 struct AsmPlan {
     AsmParams P;
+    // Inner cells, whose unknown leaves all lie in the assignable range: every such leaf has bias 0, and
+    // where the program makes of these zeros and constants nothing but (a multiple of +-1 of) one known
+    // field's value, the right-hand side there is rhs_sign x that field at offset rhs_off (rhs_sign 0: 0)
+    bool rhs_plain = false;
+    int rhs_slot = 0, rhs_off[3] = {0, 0, 0};
+    double rhs_sign = 0.;
+    Box inner;
     std::vector<PInstr> prog;
     std::vector<std::array<int, 3>> comm;  // middle cell's stencil keys, offset form, insertion order
     long long cells = 0;
