@@ -21,12 +21,12 @@ struct LvlDev {
     int gh_lo[3], gh_hi[3];  // prolongation ghost rule per side (GhostRule)
     int node;            // 1: node-centred transfers (coarse I <-> fine 2I), 0: cell-centred (I <-> 2I, 2I+1)
     int table;           // 1: coefficients from the class table, 0: SoA arrays
-    int uoff;            // 1 (2D class tables): every off-diagonal coefficient of an existing neighbour equals the
+    int uoff;            // 1 (class tables): every off-diagonal coefficient of an existing neighbour equals the
                          // interior class's, so the classes differ in the centre one only
     int rbgs;            // 1: red-black Gauss-Seidel, 0: damped Jacobi
     int problem;         // owning problem
     int coarsest;        // 1 if no coarser level
-    int tiled;           // 1: smoothed by the fused tile kernels (which also restrict into the next level)
+    int tiled;           // 1: run by the fused 2D or 3D kernels (which also restrict into the next level)
     int nslot;           // 2*ndim + 1
     const double* A64;   // [NSLOT][N]
     const float* A32;

@@ -44,6 +44,12 @@ bool mg_tiles_supported(int sweeps);
 void mg_strips(int li, const LvlDev& D, bool coarse_node, int sweeps, int rows, std::vector<Chunk>& out);
 int mg_launch_tile_down(cudaStream_t s, const LvlDev* L, const Chunk* strips, int n, const Scal* sc, int pre, int post);
 int mg_launch_tile_up(cudaStream_t s, const LvlDev* L, const Chunk* strips, int n, const Scal* sc, int pre, int post);
+// fused 3D steps of a float32 level (mg_vol.cu), as the 2D strips: one CTA per tile Chunk{lvl, j = first row,
+// k = first plane, i0 = first column, cnt = columns, nrows = planes} of mg_vol_tiles (choice: 4, or 2, 8, 16
+// for other plane counts)
+bool mg_vol_supported(int pre, int post);
+void mg_vol_tiles(int li, const LvlDev& D, int sweeps, int sms, int choice, std::vector<Chunk>& out);
+int mg_launch_vol(cudaStream_t s, const LvlDev* L, const Chunk* tiles, int n, const Scal* sc, int sweeps, bool down);
 // the V-cycle at and below each listed level of 2D problems whose levels there all take strips and whose
 // coarsest level has a dense inverse (pre = post = sweeps)
 constexpr int MG_BSTRIP_WARPS = 16, MG_BSTRIP_ROWS = 4;

@@ -335,14 +335,14 @@ static int compress_level(MGSystem* S, LevelHost& L) {
     L.table = hb == 0;
     L.tab = tab;
     // (the float32 values decide: the strips that use it run the float32 V-cycle)
-    L.uoff = L.table && L.ndim == 2;
-    for (int cls = 0; L.uoff && cls < 9; ++cls) {
-        const int c[2] = {cls % 3, cls / 3};
-        for (int d = 0; d < 2; ++d)
+    L.uoff = L.table && L.ndim >= 2;
+    for (int cls = 0, inner = L.ndim == 2 ? 4 : 13; L.uoff && cls < (L.ndim == 2 ? 9 : 27); ++cls) {
+        const int c[3] = {cls % 3, cls / 3 % 3, cls / 9};
+        for (int d = 0; d < L.ndim; ++d)
             for (int sd = 0; sd < 2; ++sd) {
                 const int q = 1 + 2 * d + sd;
                 const bool exists = L.per[d] || c[d] != (sd ? 2 : 0);
-                if (exists && t8f[cls * TSTRIDE + q] != t8f[4 * TSTRIDE + q]) L.uoff = false;
+                if (exists && t8f[cls * TSTRIDE + q] != t8f[inner * TSTRIDE + q]) L.uoff = false;
             }
     }
     if (!L.table) {
@@ -605,7 +605,7 @@ static std::string level_key(const char* kernel, const MGSystem* S, int l) {
 static int tune_levels(MGSystem* S) {
     if (!tune_enabled()) return OPFLOW_OK;
     bool any = false;
-    for (int l = 0; l < S->nlevels; ++l) any = any || S->d_zsm[l].n > 0 || !S->tile_alt[l].empty();
+    for (int l = 0; l < S->nlevels; ++l) any = any || S->d_zsm[l].n > 0 || S->d_vol[l].n > 0 || !S->tile_alt[l].empty();
     if (!any) return OPFLOW_OK;
     opflow_ctx ctx = S->ctx;
     const bool f32 = S->precision == OPFLOW_PREC_MIXED;
@@ -630,6 +630,43 @@ static int tune_levels(MGSystem* S) {
                     return smooth_z_level(S, l, 1, nullptr, zb);
                 });
             });
+        }
+        if (Z.n == 0 && S->d_vol[l].n > 0) {
+            // planes per tile of the fused 3D step (both legs timed)
+            std::map<int, std::pair<std::vector<Chunk>, ChunkList>> alt;
+            auto list = [&](int c) -> const ChunkList* {
+                if (c == 4) return &S->d_vol[l];
+                auto& e = alt[c];
+                if (!e.second.ptr) {
+                    int last = -1;
+                    for (const Chunk& t : S->vol_ch[l])
+                        if (t.lvl != last) {
+                            mg_vol_tiles(t.lvl, S->lv_host[t.lvl], S->pre, ctx->num_sms, c, e.first);
+                            last = t.lvl;
+                        }
+                    e.second.n = (int) e.first.size();
+                    e.second.ptr = (Chunk*) S->arena.alloc(e.first.size() * sizeof(Chunk));
+                    if (!e.second.ptr || cudaMemcpyAsync(e.second.ptr, e.first.data(), e.first.size() * sizeof(Chunk), cudaMemcpyHostToDevice,
+                                                         ctx->stream) != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+                        return nullptr;
+                }
+                return &e.second;
+            };
+            const int pick = choose(level_key("mg_smooth_z", S, l), {4, 2, 8, MG_ZB_TMA}, [&](int c) {
+                const ChunkList* T = list(c);
+                if (!T) return -1.f;
+                return time_launch(S, [&] {
+                    OPG_TRY(mg_launch_vol(ctx->stream, S->dL, T->ptr, T->n, nullptr, S->pre, true));
+                    return mg_launch_vol(ctx->stream, S->dL, T->ptr, T->n, nullptr, S->post, false);
+                });
+            });
+            if (pick != 4) {
+                const ChunkList* T = list(pick);
+                if (!T) return fail(OPFLOW_E_NOMEM, "tile list");
+                const ChunkList chosen = *T;
+                S->vol_ch[l].swap(alt[pick].first);
+                S->d_vol[l] = chosen;
+            }
         }
         if (!S->tile_alt[l].empty()) {
             // candidate 0: the list built (the shape the SM-fill rule picked), 1: the other shape
@@ -675,6 +712,7 @@ int mg_finalize(MGSystem* S) {
     S->restrict_ch.assign(S->nlevels, {});
     S->prolong_ch.assign(S->nlevels, {});
     S->tile_ch.assign(S->nlevels, {});
+    S->vol_ch.assign(S->nlevels, {});
     S->zsm_ch.assign(S->nlevels, {});
     S->zb.assign(S->nlevels, 4);
     S->tile_alt.assign(S->nlevels, {});
@@ -792,7 +830,16 @@ int mg_finalize(MGSystem* S) {
             for (size_t l = sp; l < P.levels.size(); ++l) bcells += P.levels[l].N;
             if (bcells > MG_BOTTOM_CELLS || P.levels.size() - sp > (size_t) MG_BOTTOM_LEVELS) sp = P.levels.size();  // chunked instead
         }
-        auto tileable = [&](size_t l) { return l < sp && stripable(l); };
+        // 3D: cell-centred, not periodic, classes that differ in the centre coefficient only
+        auto volable = [&](size_t l) {
+            if (!f32 || zoff || !mg_vol_supported(S->pre, S->post) || l >= sp || l + 1 >= P.levels.size()) return false;
+            const LevelHost &F = P.levels[l], &Cn = P.levels[l + 1];
+            if (F.ndim != 3 || !F.table || !F.uoff || F.node || Cn.node) return false;
+            for (int d = 0; d < 3; ++d)
+                if (F.per[d] || F.n[d] < 4 || Cn.n[d] != (F.n[d] + 1) / 2) return false;
+            return true;
+        };
+        auto tileable = [&](size_t l) { return (l < sp && stripable(l)) || volable(l); };
         for (size_t l = 0; l < P.levels.size(); ++l) {
             LevelHost& H = P.levels[l];
             LvlDev D{};
@@ -844,7 +891,9 @@ int mg_finalize(MGSystem* S) {
             }
             if (l >= sp) continue;                                   // inside the bottom kernel
             const bool above_tiled = l > 0 && tileable(l - 1);      // restricted by the finer level's tiles
-            if (D.tiled) {
+            if (volable(l)) {
+                mg_vol_tiles(li, D, S->pre, ctx->num_sms, 4, S->vol_ch[l]);
+            } else if (D.tiled) {
                 const bool cnode = P.levels[l + 1].node;
                 const int rows = strip_rows(l);
                 mg_strips(li, D, cnode, std::max(S->pre, S->post), rows, S->tile_ch[l]);
@@ -968,6 +1017,7 @@ int mg_finalize(MGSystem* S) {
     S->d_restrict.assign(S->nlevels, {});
     S->d_prolong.assign(S->nlevels, {});
     S->d_tiles.assign(S->nlevels, {});
+    S->d_vol.assign(S->nlevels, {});
     S->d_zsm.assign(S->nlevels, {});
     S->d_zt.assign(S->nlevels, {});
     for (int l = 0; l < S->nlevels; ++l) {
@@ -975,6 +1025,7 @@ int mg_finalize(MGSystem* S) {
         upload(S->restrict_ch[l], S->d_restrict[l]);
         upload(S->prolong_ch[l], S->d_prolong[l]);
         upload(S->tile_ch[l], S->d_tiles[l]);
+        upload(S->vol_ch[l], S->d_vol[l]);
         upload(S->zsm_ch[l], S->d_zsm[l]);
         upload(S->zt_ch[l], S->d_zt[l]);
     }
@@ -1026,6 +1077,7 @@ static int vcycle(MGSystem* S) {
     for (int l = 0; l < S->nlevels; ++l) {
         if (l > 0) OPG_TRY(mg_launch_restrict(s, sms, f32, S->dL, S->d_restrict[l].ptr, S->d_restrict[l].n, sc));
         OPG_TRY(mg_launch_tile_down(s, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->pre, S->post));
+        OPG_TRY(mg_launch_vol(s, S->dL, S->d_vol[l].ptr, S->d_vol[l].n, sc, S->pre, true));
         const ChunkList& C = S->d_smooth[l];
         const ChunkList& Z = S->d_zsm[l];
         for (int it = 0; it < S->pre; ++it) {
@@ -1046,6 +1098,7 @@ static int vcycle(MGSystem* S) {
     }
     for (int l = S->nlevels - 2; l >= 0; --l) {
         OPG_TRY(mg_launch_tile_up(s, S->dL, S->d_tiles[l].ptr, S->d_tiles[l].n, sc, S->pre, S->post));
+        OPG_TRY(mg_launch_vol(s, S->dL, S->d_vol[l].ptr, S->d_vol[l].n, sc, S->post, false));
         const ChunkList& C = S->d_smooth[l];
         const ChunkList& Z = S->d_zsm[l];
         OPG_TRY(mg_launch_prolong(s, sms, f32, S->dL, S->d_prolong[l].ptr, S->d_prolong[l].n, sc));
@@ -1304,6 +1357,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     C->restrict_ch.assign(C->nlevels, {});
     C->prolong_ch.assign(C->nlevels, {});
     C->tile_ch.assign(C->nlevels, {});
+    C->vol_ch.assign(C->nlevels, {});
     C->zsm_ch.assign(C->nlevels, {});
     C->zb.assign(C->nlevels, 4);
     C->tile_alt.assign(C->nlevels, {});
@@ -1342,6 +1396,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
             shift(P->restrict_ch[l], C->restrict_ch[l]);
             shift(P->prolong_ch[l], C->prolong_ch[l]);
             shift(P->tile_ch[l], C->tile_ch[l]);
+            shift(P->vol_ch[l], C->vol_ch[l]);
             shift(P->zsm_ch[l], C->zsm_ch[l]);
             shift(P->zt_ch[l], C->zt_ch[l]);
             if (P->zsm_ch[l].size() > zb_tiles[l]) {
@@ -1404,6 +1459,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     C->d_restrict.assign(C->nlevels, {});
     C->d_prolong.assign(C->nlevels, {});
     C->d_tiles.assign(C->nlevels, {});
+    C->d_vol.assign(C->nlevels, {});
     C->d_zsm.assign(C->nlevels, {});
     C->d_zt.assign(C->nlevels, {});
     for (int l = 0; l < C->nlevels; ++l) {
@@ -1411,6 +1467,7 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
         upload(C->restrict_ch[l], C->d_restrict[l]);
         upload(C->prolong_ch[l], C->d_prolong[l]);
         upload(C->tile_ch[l], C->d_tiles[l]);
+        upload(C->vol_ch[l], C->d_vol[l]);
         upload(C->zsm_ch[l], C->d_zsm[l]);
         upload(C->zt_ch[l], C->d_zt[l]);
     }

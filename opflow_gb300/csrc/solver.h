@@ -67,9 +67,10 @@ struct MGSystem {
     // coarse_sm: rows of coarsest levels that have no dense inverse (they are smoothed instead)
     std::vector<std::vector<Chunk>> smooth_ch, restrict_ch, prolong_ch;
     std::vector<ChunkList> d_smooth, d_restrict, d_prolong;
-    // tiles of the levels run by the fused 2D tile kernels (such levels are in none of the lists above)
-    std::vector<std::vector<Chunk>> tile_ch;
-    std::vector<ChunkList> d_tiles;
+    // strips and tiles of the levels run by the fused 2D and 3D kernels (such levels are in none of the
+    // lists above)
+    std::vector<std::vector<Chunk>> tile_ch, vol_ch;
+    std::vector<ChunkList> d_tiles, d_vol;
     // tiles of the 3D levels smoothed by the z-marching kernel (such levels are not in smooth_ch)
     std::vector<std::vector<Chunk>> zsm_ch;
     std::vector<ChunkList> d_zsm;
