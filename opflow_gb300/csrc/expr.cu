@@ -596,7 +596,6 @@ static int markstein_ok(opflow_ctx ctx, double h, bool* ok) {
     return OPFLOW_OK;
 }
 
-int markstein_ok_public(opflow_ctx ctx, double h, bool* ok) { return markstein_ok(ctx, h, ok); }
 
 // ======================================================================================== fast fixed point
 // Linear constant-coefficient stencil of one field in difference form:

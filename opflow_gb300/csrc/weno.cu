@@ -6,16 +6,23 @@
 // memory: one HBM read and one write of u per point per RK3 step (plus the optional stage fields).
 //
 // The periodic padding the reference refreshes between stages is the same line wrapped around, so
-// the stages read u[(i + o) mod n].  Divisions by the constants 3 and 6 use Markstein's correctly
-// rounded division by a constant (checked against IEEE division on the device before use); division
-// by a power-of-two h is an exact multiplication; everything else is the reference's operation.
+// the stages read u[(i + o) mod n].
 //
-// The kernel is float64-issue-bound: this GPU retires about two float64 instructions per clock per SM,
-// 1/64 of its float32 rate, so every float64 operation saved is time saved and integer work is nearly
-// free.  EXACT mode shares the terms that neighbouring points have in common (below) and keeps the
-// reference's six IEEE divisions per point.  FAST mode (not bit-identical) contracts the arithmetic and
-// forms the three nonlinear weights with one reciprocal.
-#include "internal.h"
+// The kernel is float64-issue-bound: this GPU retires two float64 instructions per clock per SM, 1/64 of
+// its float32 rate, so every float64 operation saved is time saved and integer work is nearly free.
+// EXACT mode saves operations that change no bit:
+//  - the terms that neighbouring points have in common are formed once (below);
+//  - x / 3, x / 6 and x / h are two operations, fma(x, c, x * c') with c + c' = 1/3, 1/6, 1/h to 106 bits,
+//    which is the correctly rounded quotient (div2_failures in stencil.cu: for 3 and 6 no significand can
+//    fail, for h the one that may is guarded); a power of two h moves the exponent field;
+//  - exact multiplications (by 2, 4, 1/4, and d / 6 = (d / 3) / 2) are folded into fused operations;
+//  - the six IEEE divisions per point are built from four reciprocals (div_rn: the three weights share
+//    their denominator).
+// 84 float64 operations per point and stage against 119 with the reference's operations one by one:
+// 16384 lines of 4096 cells 44.2 -> 35.2 ms.
+// FAST mode (not bit-identical) contracts the arithmetic and forms the three nonlinear weights with one
+// reciprocal.
+#include "stencil.h"
 
 #include <cmath>
 
@@ -26,9 +33,11 @@ struct WenoParams {
     int dim;          // direction
     int up;           // 1: D1WENO53Upwind (mirrored stencil, negated)
     double dt, h, inv_h;
-    int h_pow2;
-    int mk3, mk6;     // Markstein usable for /3 and /6
-    double r3, r6;    // RN(1/3), RN(1/6)
+    int h_pow2, h_shift;             // h is a power of two: division moves the exponent by h_shift
+    int h_two, h_guard, bad_hi, bad_lo;  // two-operation division by h, and the 52-bit fraction it leaves out
+    double h_cl;                     // RN(1/h - inv_h)
+    double r3, r6;                   // RN(1/3), RN(1/6)
+    double cl3, cl6;                 // RN(1/3 - r3), RN(1/6 - r6)
     double c1312, third, two_third;
     // FAST mode only: RN(5/6), RN(7/6), RN(11/6); differences are taken in units of dt/h (fdx) and the
     // smoothness indicators multiplied by 4, which leaves the weights unchanged and makes the stage
@@ -36,65 +45,19 @@ struct WenoParams {
     double c5_6, c7_6, c11_6, fdx, c1312x4, eps_floor4;
 };
 
-__device__ __forceinline__ double divc(double x, double c, double y, int mk) {
-    if (!mk) return __ddiv_rn(x, c);
-    const double q = __dmul_rn(x, y);
-    const double r = __fma_rn(-q, c, x);
-    return __fma_rn(r, y, q);
+// The rare sides of the divisions below, apart: of a branch within the code the compiler issues both sides
+// under predicates, and a float64 operation that is predicated off takes its time all the same.
+static __device__ __noinline__ double weno_div(double a, double b) { return __ddiv_rn(a, b); }
+static __device__ __noinline__ double weno_mul(double a, double b) { return __dmul_rn(a, b); }
+
+// Whether x is neither zero nor, with a wide margin, in the normal range: the steps below are not exact there.
+__device__ __forceinline__ bool out_of_range(double x) {
+    const int hi = __double2hiint(x);
+    return (unsigned) (((hi >> 20) & 0x7FF) - 150) > 1700u && ((hi & 0x7FFFFFFF) | __double2loint(x)) != 0;
 }
 
-// ---- per-point arithmetic, with the terms that neighbouring points share computed once ----------------
-// A thread evaluates K consecutive points of a line.  For Downwind the point i reads the six values
-// g[p..p+5] = u[i-3..i+2] (p = i - i0); for Upwind the mirrored values u[i+3..i-2] (the line read
-// backwards, p = i0 + K - 1 - i), negated at the end.  Point p's differences d1..d5 are D[p..p+4] with
-// D[k] = (g[k+1] - g[k]) / h, so point p + 1 reuses four of them, and with them every term the
-// reference forms from one difference alone: d/3, d/6, 5d/6, 7d/6, 11d/6, 2d, 3d, 4d, d*d, and the
-// smoothness sub-term (13/12) * ((d_k - 2 d_{k+1}) + d_{k+2})^2 that s1, s2 and s3 of three consecutive
-// points share.  Each shared term is the same IEEE operation on the same operands as in the reference's
-// kernel (D1WENO53Downwind.hpp:136-154), so EXACT results stay bit-identical; divc(-d, 6) = -divc(d, 6)
-// exactly, since every step of divc is odd in its argument.  The largest of d1^2..d5^2 is taken on the
-// bit patterns (non-negative doubles order like their bits), which equals the reference's comparisons
-// for non-NaN values.
-struct DiffTerms {
-    double D, D3, D6, D56, D76, D116, M2, M3, M4;
-    long long SQ;  // bits of D * D
-    double A;      // FAST: D / 3
-};
-
-__device__ __forceinline__ double dh_of(double a, const WenoParams& P) { return P.h_pow2 ? __dmul_rn(a, P.inv_h) : __ddiv_rn(a, P.h); }
-
-template <bool FAST>
-__device__ __forceinline__ DiffTerms diff_terms(double lo, double hi, const WenoParams& P) {
-    DiffTerms t;
-    t.D = FAST ? __dmul_rn(__dsub_rn(hi, lo), P.fdx) : dh_of(__dsub_rn(hi, lo), P);
-    t.SQ = __double_as_longlong(__dmul_rn(t.D, t.D));
-    if constexpr (FAST) t.A = __dmul_rn(P.r3, t.D);
-    if constexpr (!FAST) {
-        t.D3 = divc(t.D, 3., P.r3, P.mk3);
-        t.D6 = divc(t.D, 6., P.r6, P.mk6);
-        t.D56 = divc(__dmul_rn(5., t.D), 6., P.r6, P.mk6);
-        t.D76 = divc(__dmul_rn(7., t.D), 6., P.r6, P.mk6);
-        t.D116 = divc(__dmul_rn(11., t.D), 6., P.r6, P.mk6);
-        t.M2 = __dmul_rn(2., t.D);
-        t.M3 = __dmul_rn(3., t.D);
-        t.M4 = __dmul_rn(4., t.D);
-    }
-    return t;
-}
-
-// (13/12) * t1^2 with t1 = (d_k - 2 d_{k+1}) + d_{k+2} (FAST: 4 times that)
-template <bool FAST>
-__device__ __forceinline__ double smooth_p1(const DiffTerms& a, const DiffTerms& b, const DiffTerms& c, const WenoParams& P) {
-    if constexpr (FAST) {
-        const double t1 = __dadd_rn(__fma_rn(-2., b.D, a.D), c.D);
-        return __dmul_rn(__dmul_rn(P.c1312x4, t1), t1);
-    } else {
-        const double t1 = __dadd_rn(__dsub_rn(a.D, b.M2), c.D);
-        return __dmul_rn(P.c1312, __dmul_rn(t1, t1));
-    }
-}
-
-__device__ __forceinline__ long long max_bits(long long a, long long b) { return a < b ? b : a; }
+// correctly rounded x / c for the c whose reciprocal is ch + cl, x in range
+__device__ __forceinline__ double div_const(double x, double ch, double cl) { return __fma_rn(x, ch, __dmul_rn(x, cl)); }
 
 // 1/x for x in the normal range: the hardware's approximate reciprocal refined by the cubic Newton step
 // y = r + r*(e + e^2), e = 1 - x*r (Newton-Raphson iteration for 1/x with the second-order term; the
@@ -106,6 +69,98 @@ __device__ __forceinline__ double recip_fast(double x) {
     return __fma_rn(__fma_rn(e, e, e), r, r);
 }
 
+// a / b, correctly rounded, given y = 1/b to within an ulp (recip_fast): q = a y, the exact remainder
+// r = a - q b, and q + r y (the division steps of Markstein, IBM J. Res. Dev. 34 (1990)).  q is off a / b
+// by less than 1.5 ulps of q and y by 2^-52 of 1/b, so q + r y is off a / b by less than 2^-51 ulp before its
+// rounding; it is rounded to a / b's neighbour unless a / b lies that near the middle of two numbers.  That
+// is looked for on the bits (integer operations): |r| near ulp(q) b / 2 or 3 ulp(q) b / 2, or q next to a
+// power of two (below it the numbers are denser); then, and where an exponent is near the ends of the
+// range, the warp's lanes concerned divide.
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    const double r = __fma_rn(-q, b, a);
+    double v = __fma_rn(r, y, q);
+    const unsigned long long ab = (unsigned long long) __double_as_longlong(a), bb = (unsigned long long) __double_as_longlong(b),
+                             qb = (unsigned long long) __double_as_longlong(q), rb = (unsigned long long) __double_as_longlong(r) & 0x7FFFFFFFFFFFFFFFull;
+    const unsigned ea = (unsigned) (ab >> 52), eb = (unsigned) (bb >> 52), eq = (unsigned) (qb >> 52);  // (a, b >= 0: a sign bit fails the range test)
+    bool bad = ea - 200u > 1600u || eb - 200u > 1600u || eq - 200u > 1600u;
+    bad |= (qb & 0xFFFFFFFFFFFFFull) < 3;
+    // T = ulp(q) b / 2
+    const unsigned long long T = bb + ((unsigned long long) eq << 52) - ((unsigned long long) (1023 + 53) << 52);
+    bad |= rb - T + 64 <= 128;
+    // |r| against 3 T: significands 2^k m(r) and 3 m(b), k the difference of the exponents
+    const int k = (int) (rb >> 52) - (int) (T >> 52);
+    const unsigned long long mr = ((rb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << (k & 3), mb = 3 * ((bb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull);
+    bad |= (k == 1 || k == 2) && mr - mb + 256 <= 512;
+    if (bad) v = weno_div(a, b);
+    return v;
+}
+
+// ---- per-point arithmetic, with the terms that neighbouring points share computed once ----------------
+// A thread evaluates K consecutive points of a line.  For Downwind the point i reads the six values
+// g[p..p+5] = u[i-3..i+2] (p = i - i0); for Upwind the mirrored values u[i+3..i-2] (the line read
+// backwards, p = i0 + K - 1 - i), negated at the end.  Point p's differences d1..d5 are D[p..p+4] with
+// D[k] = (g[k+1] - g[k]) / h, so point p + 1 reuses four of them, and with them every term the
+// reference forms from one difference alone: d/3, 5d/6, 7d/6, 11d/6, 3d, d*d, and the
+// smoothness sub-term (13/12) * ((d_k - 2 d_{k+1}) + d_{k+2})^2 that s1, s2 and s3 of three consecutive
+// points share.  Each shared term is the same IEEE operation on the same operands as in the reference's
+// kernel (D1WENO53Downwind.hpp:136-154), so EXACT results stay bit-identical.  The largest of d1^2..d5^2 is taken on the
+// bit patterns (non-negative doubles order like their bits), which equals the reference's comparisons
+// for non-NaN values.
+struct DiffTerms {
+    double D, D3, D56, D76, D116, M3;
+    long long SQ;  // bits of D * D
+    double A;      // FAST: D / 3
+};
+
+__device__ __forceinline__ double dh_of(double a, const WenoParams& P) {
+    const int hi = __double2hiint(a), lo = __double2loint(a);
+    if (P.h_pow2) {
+        // exponent arithmetic for normal operands and quotients; zeros stay
+        const int e = (hi >> 20) & 0x7FF;
+        const bool zero = ((hi & 0x7FFFFFFF) | lo) == 0;
+        double r = __hiloint2double(zero ? hi : hi + P.h_shift * (1 << 20), lo);
+        if (!zero && ((unsigned) (e - 1) >= 2046u || (unsigned) (e + P.h_shift - 1) >= 2046u)) r = weno_mul(a, P.inv_h);
+        return r;
+    }
+    if (!P.h_two) return weno_div(a, P.h);
+    double r = div_const(a, P.inv_h, P.h_cl);
+    if (out_of_range(a) || (P.h_guard && lo == P.bad_lo && (hi & 0xFFFFF) == P.bad_hi)) r = weno_div(a, P.h);
+    return r;
+}
+
+template <bool FAST>
+__device__ __forceinline__ DiffTerms diff_terms(double lo, double hi, const WenoParams& P) {
+    DiffTerms t;
+    t.D = FAST ? __dmul_rn(__dsub_rn(hi, lo), P.fdx) : dh_of(__dsub_rn(hi, lo), P);
+    t.SQ = __double_as_longlong(__dmul_rn(t.D, t.D));
+    if constexpr (FAST) t.A = __dmul_rn(P.r3, t.D);
+    if constexpr (!FAST) {
+        t.D3 = div_const(t.D, P.r3, P.cl3);
+        t.D56 = div_const(__dmul_rn(5., t.D), P.r6, P.cl6);
+        t.D76 = div_const(__dmul_rn(7., t.D), P.r6, P.cl6);
+        t.D116 = div_const(__dmul_rn(11., t.D), P.r6, P.cl6);
+        if (out_of_range(t.D)) {
+            t.D3 = weno_div(t.D, 3.);
+            t.D56 = weno_div(weno_mul(5., t.D), 6.);
+            t.D76 = weno_div(weno_mul(7., t.D), 6.);
+            t.D116 = weno_div(weno_mul(11., t.D), 6.);
+        }
+        t.M3 = __dmul_rn(3., t.D);
+    }
+    return t;
+}
+
+// (13/12) * t1^2 with t1 = (d_k - 2 d_{k+1}) + d_{k+2} (FAST: 4 times that)
+template <bool FAST>
+__device__ __forceinline__ double smooth_p1(const DiffTerms& a, const DiffTerms& b, const DiffTerms& c, const WenoParams& P) {
+    const double t1 = __dadd_rn(__fma_rn(-2., b.D, a.D), c.D);  // (2 d is exact)
+    if constexpr (FAST) return __dmul_rn(__dmul_rn(P.c1312x4, t1), t1);
+    else return __dmul_rn(P.c1312, __dmul_rn(t1, t1));
+}
+
+__device__ __forceinline__ long long max_bits(long long a, long long b) { return a < b ? b : a; }
+
 // the WENO5-JS derivative at point p from the five difference windows X0..X4 (= D[p..p+4]) and the three
 // smoothness sub-terms of windows p, p+1, p+2 (FAST: dt times the derivative)
 template <bool FAST>
@@ -114,22 +169,23 @@ __device__ __forceinline__ double weno_point(const DiffTerms& X0, const DiffTerm
     long long mb = max_bits(max_bits(max_bits(X0.SQ, X1.SQ), max_bits(X2.SQ, X3.SQ)), X4.SQ);
     const double mx = __longlong_as_double(mb);
     if constexpr (!FAST) {
+        // (d / 6 = (d / 3) / 2, 4 d and t / 4 are exact: folded into the operation that takes them)
         const double ddx1 = __dadd_rn(__dsub_rn(X0.D3, X1.D76), X2.D116);
-        const double ddx2 = __dadd_rn(__dadd_rn(-X1.D6, X2.D56), X3.D3);
-        const double ddx3 = __dsub_rn(__dadd_rn(X2.D3, X3.D56), X4.D6);
-        double t2 = __dadd_rn(__dsub_rn(X0.D, X1.M4), X2.M3);
-        const double s1 = __dadd_rn(p0, __dmul_rn(__dmul_rn(t2, t2), 0.25));
+        const double ddx2 = __dadd_rn(__fma_rn(-0.5, X1.D3, X2.D56), X3.D3);
+        const double ddx3 = __fma_rn(-0.5, X4.D3, __dadd_rn(X2.D3, X3.D56));
+        double t2 = __dadd_rn(__fma_rn(-4., X1.D, X0.D), X2.M3);
+        const double s1 = __fma_rn(0.25, __dmul_rn(t2, t2), p0);
         t2 = __dsub_rn(X1.D, X3.D);
-        const double s2 = __dadd_rn(p1, __dmul_rn(__dmul_rn(t2, t2), 0.25));
-        t2 = __dadd_rn(__dsub_rn(X2.M3, X3.M4), X4.D);
-        const double s3 = __dadd_rn(p2, __dmul_rn(__dmul_rn(t2, t2), 0.25));
+        const double s2 = __fma_rn(0.25, __dmul_rn(t2, t2), p1);
+        t2 = __dadd_rn(__fma_rn(-4., X3.D, X2.M3), X4.D);
+        const double s3 = __fma_rn(0.25, __dmul_rn(t2, t2), p2);
         const double eps = __dadd_rn(__dmul_rn(1e-6, mx), 1e-99);
         double q;
-        q = __dadd_rn(s1, eps); const double a1 = __ddiv_rn(.1, __dmul_rn(q, q));
-        q = __dadd_rn(s2, eps); const double a2 = __ddiv_rn(.6, __dmul_rn(q, q));
-        q = __dadd_rn(s3, eps); const double a3 = __ddiv_rn(.3, __dmul_rn(q, q));
-        const double sum = __dadd_rn(__dadd_rn(a1, a2), a3);
-        const double w1 = __ddiv_rn(a1, sum), w2 = __ddiv_rn(a2, sum), w3 = __ddiv_rn(a3, sum);
+        q = __dadd_rn(s1, eps); q = __dmul_rn(q, q); const double a1 = div_rn(.1, q, recip_fast(q));
+        q = __dadd_rn(s2, eps); q = __dmul_rn(q, q); const double a2 = div_rn(.6, q, recip_fast(q));
+        q = __dadd_rn(s3, eps); q = __dmul_rn(q, q); const double a3 = div_rn(.3, q, recip_fast(q));
+        const double sum = __dadd_rn(__dadd_rn(a1, a2), a3), y = recip_fast(sum);
+        const double w1 = div_rn(a1, sum, y), w2 = div_rn(a2, sum, y), w3 = div_rn(a3, sum, y);
         return __dadd_rn(__dadd_rn(__dmul_rn(w1, ddx1), __dmul_rn(w2, ddx2)), __dmul_rn(w3, ddx3));
     } else {
         // The same quantities with contracted arithmetic, in the scaled units above, and one reciprocal:
@@ -208,7 +264,7 @@ __device__ __forceinline__ void weno_stage(const double* __restrict__ u, const d
             const double L = FAST ? r : __dmul_rn(P.dt, r);
             double v;
             if constexpr (STAGE == 0) v = __dsub_rn(u[i], L);
-            else if constexpr (STAGE == 1) v = __dadd_rn(__dmul_rn(0.75, u[i]), __dmul_rn(0.25, __dsub_rn(src[i], L)));
+            else if constexpr (STAGE == 1) v = __fma_rn(0.25, __dsub_rn(src[i], L), __dmul_rn(0.75, u[i]));  // (x / 4 is exact)
             else v = __dadd_rn(__dmul_rn(P.third, u[i]), __dmul_rn(P.two_third, __dsub_rn(src[i], L)));
             out[i] = v;
             X[0] = X[1];
@@ -307,8 +363,6 @@ __global__ void __launch_bounds__(kWenoThreads, MINB) weno_rk3_kernel(FieldView 
     }
 }
 
-extern int markstein_ok_public(opflow_ctx ctx, double h, bool* ok);
-
 }  // namespace opg
 
 using namespace opg;
@@ -363,17 +417,18 @@ extern "C" int opflow_weno_rk3_mode(opflow_ctx ctx, opflow_field u, opflow_field
     P.dt = dt;
     P.h = u->mesh->h[dim];
     P.inv_h = 1.0 / P.h;
-    {
-        int e;
-        P.h_pow2 = std::frexp(P.h, &e) == 0.5;
-    }
-    bool ok3 = false, ok6 = false;
-    OPG_TRY(markstein_ok_public(ctx, 3.0, &ok3));
-    OPG_TRY(markstein_ok_public(ctx, 6.0, &ok6));
-    P.mk3 = ok3;
-    P.mk6 = ok6;
+    AxisParams A{};
+    P.h_two = axis_divisor(&A, 0, P.h);
+    P.h_pow2 = P.h_two && A.pow2[0];
+    P.h_shift = A.shift[0];
+    P.h_cl = A.cl[0];
+    P.h_guard = A.guard[0];
+    P.bad_hi = A.bad_hi[0];
+    P.bad_lo = A.bad_lo[0];
     P.r3 = 1.0 / 3.0;
     P.r6 = 1.0 / 6.0;
+    P.cl3 = std::fma(-P.r3, 3.0, 1.0) / 3.0;
+    P.cl6 = std::fma(-P.r6, 6.0, 1.0) / 6.0;
     P.c1312 = 13. / 12.;
     P.third = 1.0 / 3.0;
     P.two_third = 2.0 / 3.0;
