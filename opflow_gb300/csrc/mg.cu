@@ -6,6 +6,7 @@
 // problem in a fixed order, so a problem's iterates are bit-identical whether it runs alone or in a
 // batch.  T selects the precision of the V-cycle (float for the mixed form, double for the plain one);
 // the Krylov vectors, their updates and all inner products are float64.
+#include "f32bits.h"
 #include "mg_device.h"
 #include "tma.h"
 
@@ -665,19 +666,84 @@ __global__ void __launch_bounds__(512) mg_bottom(const LvlDev* __restrict__ Ls, 
 }
 
 // ------------------------------------------------------------------------------------ Krylov (FP64)
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    // fixed-order reduction: warp tree, then warp 0 over the warp sums
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    double t = 0.;
-    if (w == 0) {
-        t = l < (int) (blockDim.x >> 5) ? sh[l] : 0.;
-        for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+// Conversions of the streaming kernels below by integer operations (f32bits.h); zeros of either sign and
+// normal numbers on both sides, the rest in functions of their own: a conversion instruction takes the
+// float64 pipe's time even where it is predicated off.  With the shorter sums (warp_sum_256), 256^3:
+// kr_from_vcycle 125 -> 84 us, kr_pupdate 77 -> 48, kr_update 179 -> 162 (its bytes: 138).
+static __device__ __noinline__ double widen_apart(float v) { return (double) v; }
+static __device__ __noinline__ float narrow_apart(double v) { return (float) v; }
+__device__ __forceinline__ double widen(float v) {
+    const Bits64 w = f32_to_f64_bits(__float_as_uint(v));
+    return __hiloint2double((int) w.hi, (int) w.lo);
+}
+__device__ __forceinline__ float narrow(double v) { return __uint_as_float(f64_to_f32_bits((uint32_t) __double2hiint(v), (uint32_t) __double2loint(v))); }
+__device__ __forceinline__ bool plain(float v) { return f32_plain(__float_as_uint(v)); }
+__device__ __forceinline__ bool plain(double v) { return f64_plain((uint32_t) __double2hiint(v), (uint32_t) __double2loint(v)); }
+// a pair of the V-cycle's type T from / to float64
+template <typename T>
+struct Pair;
+template <>
+struct Pair<float> {
+    using V = float2;
+    __device__ __forceinline__ static V make(double a, double b) {
+        float2 v = make_float2(narrow(a), narrow(b));
+        if (!(plain(a) && plain(b))) v = make_float2(narrow_apart(a), narrow_apart(b));
+        return v;
     }
-    return t;  // valid in thread 0
+    __device__ __forceinline__ static double2 wide(float2 v) {
+        double2 w = make_double2(widen(v.x), widen(v.y));
+        if (!(plain(v.x) && plain(v.y))) w = make_double2(widen_apart(v.x), widen_apart(v.y));
+        return w;
+    }
+    __device__ __forceinline__ static float one(double a) { return plain(a) ? narrow(a) : narrow_apart(a); }
+    __device__ __forceinline__ static double wide1(float v) { return plain(v) ? widen(v) : widen_apart(v); }
+};
+template <>
+struct Pair<double> {
+    using V = double2;
+    __device__ __forceinline__ static V make(double a, double b) { return make_double2(a, b); }
+    __device__ __forceinline__ static double2 wide(double2 v) { return v; }
+    __device__ __forceinline__ static double one(double a) { return a; }
+    __device__ __forceinline__ static double wide1(double v) { return v; }
+};
+
+constexpr int KR_THREADS = 256;
+
+// Sum of sh[0 .. 255] in a fixed order (each warp's 32 values by an exchange tree of distances 16 .. 1, then
+// the eight sums by 4 .. 1), by one warp, valid in its lane 0.  The tree's additions are spread over the
+// lanes: 12 float64 warp instructions, where eight warps summing their own values take 45 (and every one
+// of them takes the float64 pipe 16 cycles).
+__device__ __forceinline__ double warp_sum_256(const double* sh) {
+    const int l = threadIdx.x & 31, h = l >> 4, m = l & 15;
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = sh[32 * (h + 2 * q) + m] + sh[32 * (h + 2 * q) + m + 16];
+    const bool u8 = (l & 8) != 0, u4 = (l & 4) != 0;
+    double a = (u8 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, u8 ? v[0] : v[1], 8);
+    const double b = (u8 ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, u8 ? v[2] : v[3], 8);
+    a = (u4 ? b : a) + __shfl_xor_sync(0xffffffffu, u4 ? a : b, 4);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    // lane l holds the sum of warp (l >> 4 & 1) + 2 (l >> 3 & 1) + 4 (l >> 2 & 1)
+    a += __shfl_xor_sync(0xffffffffu, a, 4);
+    a += __shfl_xor_sync(0xffffffffu, a, 8);
+    a += __shfl_xor_sync(0xffffffffu, a, 16);
+    return a;
+}
+
+// The CTA's sum of v (of v and w): valid in thread 0 (v) and thread 32 (w)
+__device__ __forceinline__ double block_sum(double v, double* sh) {
+    __syncthreads();
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    return threadIdx.x < 32 ? warp_sum_256(sh) : 0.;
+}
+__device__ __forceinline__ double block_sum2(double v, double w, double* sh) {
+    __syncthreads();
+    sh[threadIdx.x] = v;
+    sh[KR_THREADS + threadIdx.x] = w;
+    __syncthreads();
+    return threadIdx.x < 64 ? warp_sum_256(sh + (threadIdx.x >> 5) * KR_THREADS) : 0.;
 }
 
 // scalar steps: stage 0 after init (bb, rr), 1 after A p (pq -> alpha), 2 after the update (rr ->
@@ -708,15 +774,16 @@ __device__ __forceinline__ void scalars_stage(Scal& S, double a, double b, int s
     }
 }
 
-// Called by every thread of the CTA after thread 0 has stored chunk c's partials for problem p: the CTA
-// that completes the problem's last chunk reduces and applies the scalar stage.
-__device__ __forceinline__ void chunk_finish(const Finish& F, int p, const double* partial, double* sh, int* flag) {
+// Called by every thread of the CTA after the partials of `mine` chunks of problem p were stored (by threads
+// 0 and 32): the CTA that completes the problem's last chunk reduces and applies the scalar stage.
+__device__ __forceinline__ void chunk_finish(const Finish& F, int p, int mine, const double* partial, double* sh, int* flag) {
     if (!F.done) return;
+    if (threadIdx.x < 64) __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        const int old = atomicAdd(&F.done[p], 1);
-        *flag = old == F.count[p] - 1;
+        const int old = atomicAdd(&F.done[p], mine);
+        *flag = old + mine == F.count[p];
     }
     __syncthreads();
     if (!*flag) return;
@@ -740,56 +807,152 @@ __device__ __forceinline__ void chunk_finish(const Finish& F, int p, const doubl
 // With to_vc (mode 0) the V-cycle's level-0 input is written as well: b = (T) r, x = 0.
 // With skip0 (mode 0) the first unknown's r is left out of r.r: the true residual of a pinned system,
 // whose first row is the identity with b = 0 (satisfied exactly once the solution is shifted to x[0] = 0).
+//
+// A thread marches up to KR_SEG rows of a column, so that a row's values serve as the next row's lower
+// neighbours and the coefficients of a class-table level stay in registers.  Neighbours outside a
+// non-periodic box count as zeros.  What bounds a class-table level is the float64 pipe: 6 / 8 operations per
+// cell in 2D / 3D (256^3: 232 us at two per clock and SM); an array level reads 7 coefficients per cell.
+// Measured against a thread per cell: 256^3 302 -> 257 us, 18.5 M cells in 2D 283 -> 260, 192^3 with array
+// coefficients 304 -> 158.  The variants are functions apart, so that each has its own registers (inlined
+// they spill at four CTAs per SM).
+constexpr int KR_SEG = 8;
+
+template <typename T, int mode, int ND, bool TABLE>
+static __device__ __noinline__ double2 apply_chunk(const LvlDev& L, const KrylovDev& Kp, const Chunk C, int to_vc, int skip0) {
+    double s0 = 0., s1 = 0.;
+    const double* __restrict__ in = mode == 0 ? Kp.x : Kp.p;
+    const double* __restrict__ bp = Kp.b;
+    double* __restrict__ rp = Kp.r;
+    double* __restrict__ qp = Kp.q;
+    T* __restrict__ vb = Sel<T>::b(L);
+    T* __restrict__ vx = Sel<T>::x(L);
+    const int n0 = L.n[0], n1 = ND > 1 ? L.n[1] : 1, n2 = ND > 2 ? L.n[2] : 1, k = C.k;
+    const long long sz = (long long) n0 * n1;
+    const double* __restrict__ Tb = L.T64;
+    const double* __restrict__ A = L.A64;
+    const bool hb = ND > 2 && (k > 0 || L.per[2]), ht = ND > 2 && (k < n2 - 1 || L.per[2]);
+    const long long ob = !hb ? 0 : k > 0 ? -sz : sz * (n2 - 1), ot = !ht ? 0 : k < n2 - 1 ? sz : -sz * (n2 - 1);
+    const int zc = ND > 2 ? 9 * pos_class(k, n2) : 0;
+    const int items = C.cnt * ((C.nrows + KR_SEG - 1) / KR_SEG);
+    for (int it = threadIdx.x; it < items; it += KR_THREADS) {
+        const int sg = it / C.cnt, i = C.i0 + it - sg * C.cnt;
+        const int js = C.j + sg * KR_SEG, je = min(js + KR_SEG, C.j + C.nrows);
+        const bool hw = i > 0 || L.per[0], he = i < n0 - 1 || L.per[0];
+        const int ow = !hw ? 0 : i > 0 ? -1 : n0 - 1, oe = !he ? 0 : i < n0 - 1 ? 1 : 1 - n0;
+        long long cell = cell_of(L, i, js, k);
+        const int xz = pos_class(i, n0) + zc;
+        const double* __restrict__ p = in + cell;
+        double c = *p, lo = 0.;
+        if (ND > 1) {
+            if (js > 0) lo = *(p - n0);
+            else if (L.per[1]) lo = p[(long long) (n1 - 1) * n0];
+        }
+        // neighbours of the row at q: x and upper y (2D: loaded a row ahead)
+        auto row = [&](const double* __restrict__ q, int j, double& w, double& e, double& hi) {
+            const long long on = j < n1 - 1 ? n0 : L.per[1] ? -(long long) (n1 - 1) * n0 : 0;
+            w = q[ow];
+            e = q[oe];
+            hi = ND > 1 ? q[on] : 0.;
+            w = hw ? w : 0.;
+            e = he ? e : 0.;
+            hi = on != 0 ? hi : 0.;
+        };
+        double cf[2 * ND + 1], w, e, hi;
+        int yc = -1;
+        if (ND < 3) row(p, js, w, e, hi);
+#pragma unroll 1
+        for (int j = js; j < je; ++j, cell += n0, p += n0) {
+            const int y = ND > 1 ? pos_class(j, n1) : 0;
+            if (!TABLE) {
+#pragma unroll
+                for (int q = 0; q <= 2 * ND; ++q) cf[q] = A[(long long) q * L.N + cell];
+            } else if (y != yc) {
+                yc = y;
+#pragma unroll
+                for (int q = 0; q <= 2 * ND; ++q) cf[q] = Tb[(xz + 3 * y) * TSTRIDE + q];
+            }
+            double w1 = 0., e1 = 0., h1 = 0.;
+            if (ND == 3) row(p, j, w, e, hi);
+            else row(j + 1 < je ? p + n0 : p, min(j + 1, je - 1), w1, e1, h1);
+            const double bo = hb ? p[ob] : 0., to = ht ? p[ot] : 0.;
+            double bv = 0.;
+            if constexpr (mode == 0) bv = bp[cell];
+            double ax = cf[1] * w;
+            ax = fma(cf[2], e, ax);
+            if (ND > 1) {
+                ax = fma(cf[3], lo, ax);
+                ax = fma(cf[4], hi, ax);
+            }
+            if (ND > 2) {
+                ax = fma(cf[ND > 2 ? 5 : 0], bo, ax);
+                ax = fma(cf[ND > 2 ? 6 : 0], to, ax);
+            }
+            ax = fma(cf[0], c, ax);
+            if constexpr (mode == 0) {
+                const double r = bv - ax;
+                rp[cell] = r;
+                s0 = fma(bv, bv, s0);
+                if (!(skip0 && cell == 0)) s1 = fma(r, r, s1);
+                if (to_vc) {
+                    vb[cell] = Pair<T>::one(r);
+                    vx[cell] = 0;
+                }
+            } else {
+                qp[cell] = ax;
+                s0 = fma(c, ax, s0);
+            }
+            lo = c;
+            c = hi;
+            if (ND < 3) {
+                w = w1;
+                e = e1;
+                hi = h1;
+            }
+        }
+    }
+    return make_double2(s0, s1);
+}
+
 template <typename T, int mode>
-__global__ void __launch_bounds__(256, 4) kr_apply(const LvlDev* __restrict__ Ls, const KrylovDev* __restrict__ K, const Chunk* __restrict__ ch, int nch,
-                                                   const Scal* sc, double* partial, int to_vc, Finish F, int skip0) {
-    __shared__ double sh[32];
+__global__ void __launch_bounds__(KR_THREADS, 4) kr_apply(const LvlDev* __restrict__ Ls, const KrylovDev* __restrict__ K, const Chunk* __restrict__ ch,
+                                                          int nch, const Scal* sc, double* partial, int to_vc, Finish F, int skip0) {
+    __shared__ double sh[2 * KR_THREADS];
     __shared__ int flag;
+    int mine = 0;
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
         const Chunk C = ch[c];
         const LvlDev& L = Ls[C.lvl];
         const int pb = L.problem;
-        const bool act = !sc || sc[pb].active;
-        const KrylovDev& Kp = K[pb];
-        double s0 = 0., s1 = 0.;
-        if (act) {
-            const double* __restrict__ in = mode == 0 ? Kp.x : Kp.p;
-            const double* __restrict__ bp = Kp.b;
-            double* __restrict__ rp = Kp.r;
-            double* __restrict__ qp = Kp.q;
-            T* __restrict__ vb = Sel<T>::b(L);
-            T* __restrict__ vx = Sel<T>::x(L);
-            for (int rw = 0; rw < C.nrows; ++rw)
-#pragma unroll 2
-                for (int t = threadIdx.x; t < C.cnt; t += blockDim.x) {
-                    const int i = C.i0 + t, j = C.j + rw;
-                    const long long cell = cell_of(L, i, j, C.k);
-                    double c0, offd;
-                    stencil_parts<double>(L, in, i, j, C.k, cell, c0, offd);
-                    const double ax = fma(c0, in[cell], offd);
-                    if constexpr (mode == 0) {
-                        const double bv = bp[cell];
-                        const double r = bv - ax;
-                        rp[cell] = r;
-                        s0 = fma(bv, bv, s0);
-                        if (!(skip0 && cell == 0)) s1 = fma(r, r, s1);
-                        if (to_vc) {
-                            vb[cell] = (T) r;
-                            vx[cell] = 0;
-                        }
-                    } else {
-                        qp[cell] = ax;
-                        s0 = fma(in[cell], ax, s0);
-                    }
-                }
+        double2 s = make_double2(0., 0.);
+        if (!sc || sc[pb].active) {
+            const KrylovDev& Kp = K[pb];
+            if (L.ndim == 3) {
+                if (L.table) s = apply_chunk<T, mode, 3, true>(L, Kp, C, to_vc, skip0);
+                else s = apply_chunk<T, mode, 3, false>(L, Kp, C, to_vc, skip0);
+            } else if (L.ndim == 2) {
+                if (L.table) s = apply_chunk<T, mode, 2, true>(L, Kp, C, to_vc, skip0);
+                else s = apply_chunk<T, mode, 2, false>(L, Kp, C, to_vc, skip0);
+            } else {
+                if (L.table) s = apply_chunk<T, mode, 1, true>(L, Kp, C, to_vc, skip0);
+                else s = apply_chunk<T, mode, 1, false>(L, Kp, C, to_vc, skip0);
+            }
         }
-        const double a = block_sum(s0, sh);
-        const double b = block_sum(s1, sh);
-        if (threadIdx.x == 0) {
-            partial[2 * c] = act ? a : 0.;
-            partial[2 * c + 1] = act ? b : 0.;
+        if constexpr (mode == 0) {
+            const double a = block_sum2(s.x, s.y, sh);
+            if (threadIdx.x == 0) partial[2 * c] = a;
+            if (threadIdx.x == 32) partial[2 * c + 1] = a;
+        } else {
+            const double a = block_sum(s.x, sh);
+            if (threadIdx.x == 0) {
+                partial[2 * c] = a;
+                partial[2 * c + 1] = 0.;
+            }
         }
-        chunk_finish(F, pb, partial, sh, &flag);
+        ++mine;
+        if (c + gridDim.x >= nch || ch[c + gridDim.x].lvl != C.lvl) {
+            chunk_finish(F, pb, mine, partial, sh, &flag);
+            mine = 0;
+        }
     }
 }
 
@@ -813,25 +976,13 @@ __device__ __forceinline__ void split_run(long long start, long long n, long lon
     np = rest / 2;
     tail = (rest & 1) ? a + 2 * np : -1;
 }
-template <typename T>
-struct Pair;
-template <>
-struct Pair<float> {
-    using V = float2;
-    __device__ static V make(double a, double b) { return make_float2((float) a, (float) b); }
-};
-template <>
-struct Pair<double> {
-    using V = double2;
-    __device__ static V make(double a, double b) { return make_double2(a, b); }
-};
-
 // x += alpha p, r -= alpha q, partial (r.r); the V-cycle's level-0 input b = (T) r, x = 0 alongside
 template <typename T>
 __global__ void __launch_bounds__(256, 4) kr_update(const LvlDev* __restrict__ Ls, const KrylovDev* __restrict__ K, const Chunk* __restrict__ ch, int nch,
                                                  const Scal* sc, double* partial, Finish F) {
-    __shared__ double sh[32];
+    __shared__ double sh[KR_THREADS];
     __shared__ int flag;
+    int mine = 0;
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
         const Chunk C = ch[c];
         const LvlDev& L = Ls[C.lvl];
@@ -857,7 +1008,7 @@ __global__ void __launch_bounds__(256, 4) kr_update(const LvlDev* __restrict__ L
                     const double r = fma(-al, qp[cell], rp[cell]);
                     rp[cell] = r;
                     s = fma(r, r, s);
-                    vb[cell] = (T) r;
+                    vb[cell] = Pair<T>::one(r);
                     vx[cell] = 0;
                 };
                 if (head >= 0 && threadIdx.x == 0) one(head);
@@ -882,7 +1033,7 @@ __global__ void __launch_bounds__(256, 4) kr_update(const LvlDev* __restrict__ L
                     s = fma(rv.x, rv.x, s);
                     s = fma(rv.y, rv.y, s);
                     b2[t] = Pair<T>::make(rv.x, rv.y);
-                    z2[t] = Pair<T>::make(0., 0.);
+                    z2[t] = V{0, 0};
                 }
             } else {
                 for (int rw = 0; rw < C.nrows; ++rw)
@@ -893,14 +1044,21 @@ __global__ void __launch_bounds__(256, 4) kr_update(const LvlDev* __restrict__ L
                         const double r = fma(-al, qp[cell], rp[cell]);
                         rp[cell] = r;
                         s = fma(r, r, s);
-                        vb[cell] = (T) r;
+                        vb[cell] = Pair<T>::one(r);
                         vx[cell] = 0;
                     }
             }
         }
         const double a = block_sum(s, sh);
-        if (threadIdx.x == 0) { partial[2 * c] = act ? a : 0.; partial[2 * c + 1] = 0.; }
-        chunk_finish(F, pb, partial, sh, &flag);
+        if (threadIdx.x == 0) {
+            partial[2 * c] = a;
+            partial[2 * c + 1] = 0.;
+        }
+        ++mine;
+        if (c + gridDim.x >= nch || ch[c + gridDim.x].lvl != C.lvl) {
+            chunk_finish(F, pb, mine, partial, sh, &flag);
+            mine = 0;
+        }
     }
 }
 
@@ -908,8 +1066,9 @@ __global__ void __launch_bounds__(256, 4) kr_update(const LvlDev* __restrict__ L
 template <typename T>
 __global__ void __launch_bounds__(256, 4) kr_from_vcycle(const LvlDev* __restrict__ Ls, const KrylovDev* __restrict__ K, const Chunk* __restrict__ ch,
                                                       int nch, const Scal* sc, double* partial, Finish F) {
-    __shared__ double sh[32];
+    __shared__ double sh[2 * KR_THREADS];
     __shared__ int flag;
+    int mine = 0;
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
         const Chunk C = ch[c];
         const LvlDev& L = Ls[C.lvl];
@@ -926,7 +1085,7 @@ __global__ void __launch_bounds__(256, 4) kr_from_vcycle(const LvlDev* __restric
                 long long a0, np, head, tail;
                 split_run(st, n, a0, np, head, tail);
                 auto one = [&](long long cell) {
-                    const double z = (double) x[cell];
+                    const double z = Pair<T>::wide1(x[cell]);
                     s0 = fma(z, rp[cell], s0);
                     s1 = fma(z, qp[cell], s1);
                 };
@@ -938,28 +1097,31 @@ __global__ void __launch_bounds__(256, 4) kr_from_vcycle(const LvlDev* __restric
 #pragma unroll 4
                 for (long long t = threadIdx.x; t < np; t += blockDim.x) {
                     const V zv = z2[t];
-                    const double2 rv = r2[t], qv = q2[t];
-                    const double za = (double) zv.x, zb = (double) zv.y;
-                    s0 = fma(za, rv.x, s0);
-                    s1 = fma(za, qv.x, s1);
-                    s0 = fma(zb, rv.y, s0);
-                    s1 = fma(zb, qv.y, s1);
+                    const double2 rv = r2[t], qv = q2[t], z = Pair<T>::wide(zv);
+                    s0 = fma(z.x, rv.x, s0);
+                    s1 = fma(z.x, qv.x, s1);
+                    s0 = fma(z.y, rv.y, s0);
+                    s1 = fma(z.y, qv.y, s1);
                 }
             } else {
                 for (int rw = 0; rw < C.nrows; ++rw)
 #pragma unroll 4
                     for (int t = threadIdx.x; t < C.cnt; t += blockDim.x) {
                         const long long cell = cell_of(L, C.i0 + t, C.j + rw, C.k);
-                        const double z = (double) x[cell];
+                        const double z = Pair<T>::wide1(x[cell]);
                         s0 = fma(z, rp[cell], s0);
                         s1 = fma(z, qp[cell], s1);
                     }
             }
         }
-        const double a = block_sum(s0, sh);
-        const double b = block_sum(s1, sh);
-        if (threadIdx.x == 0) { partial[2 * c] = act ? a : 0.; partial[2 * c + 1] = act ? b : 0.; }
-        chunk_finish(F, L.problem, partial, sh, &flag);
+        const double a = block_sum2(s0, s1, sh);
+        if (threadIdx.x == 0) partial[2 * c] = a;
+        if (threadIdx.x == 32) partial[2 * c + 1] = a;
+        ++mine;
+        if (c + gridDim.x >= nch || ch[c + gridDim.x].lvl != C.lvl) {
+            chunk_finish(F, L.problem, mine, partial, sh, &flag);
+            mine = 0;
+        }
     }
 }
 
@@ -992,7 +1154,7 @@ __global__ void __launch_bounds__(256) kr_pupdate(const LvlDev* __restrict__ Ls,
             long long a0, np, head, tail;
             split_run(st, n, a0, np, head, tail);
             auto one = [&](long long cell) {
-                const double z = (double) x[cell];
+                const double z = Pair<T>::wide1(x[cell]);
                 pp[cell] = first ? z : fma(be, pp[cell], z);
             };
             if (head >= 0 && threadIdx.x == 0) one(head);
@@ -1002,21 +1164,19 @@ __global__ void __launch_bounds__(256) kr_pupdate(const LvlDev* __restrict__ Ls,
 #pragma unroll 4
             for (long long t = threadIdx.x; t < np; t += blockDim.x) {
                 const V zv = z2[t];
-                double2 pv;
-                if (first) pv = make_double2((double) zv.x, (double) zv.y);
-                else {
-                    pv = p2[t];
-                    pv.x = fma(be, pv.x, (double) zv.x);
-                    pv.y = fma(be, pv.y, (double) zv.y);
-                }
-                p2[t] = pv;
+                double2 pv = make_double2(0., 0.);
+                if (!first) pv = p2[t];
+                const double2 z = Pair<T>::wide(zv);
+                pv.x = fma(be, pv.x, z.x);
+                pv.y = fma(be, pv.y, z.y);
+                p2[t] = first ? z : pv;
             }
         } else {
             for (int rw = 0; rw < C.nrows; ++rw)
 #pragma unroll 4
                 for (int t = threadIdx.x; t < C.cnt; t += blockDim.x) {
                     const long long cell = cell_of(L, C.i0 + t, C.j + rw, C.k);
-                    const double z = (double) x[cell];
+                    const double z = Pair<T>::wide1(x[cell]);
                     pp[cell] = first ? z : fma(be, pp[cell], z);
                 }
         }
@@ -1026,7 +1186,7 @@ __global__ void __launch_bounds__(256) kr_pupdate(const LvlDev* __restrict__ Ls,
 // per-problem sums of the chunk partials, in chunk order: out[2*p + s] = sum over the problem's chunks
 __global__ void __launch_bounds__(256) kr_reduce(const double* __restrict__ partial, const int* __restrict__ first, const int* __restrict__ count,
                                                  int nprob, double* out) {
-    __shared__ double sh[32];
+    __shared__ double sh[KR_THREADS];
     for (int p = blockIdx.x; p < nprob; p += gridDim.x) {
         for (int s = 0; s < 2; ++s) {
             double v = 0.;
