@@ -2,6 +2,7 @@
 // (mg.cu) and the tile kernels (mg_tiles.cu): operator access and the per-cell bodies of smoothing,
 // residual, restriction and prolongation.
 #pragma once
+#include "f64div.h"
 #include "mg_kernels.h"
 
 namespace opg {
@@ -99,7 +100,52 @@ __device__ __forceinline__ void cell_gs(const LvlDev& L, int i, int j, int k) {
     int cls;
     stencil_parts<T>(L, x, i, j, k, cell, c0, offd, &cls);
     const T num = Sel<T>::b(L)[cell] - offd;
-    x[cell] = L.table ? num * Sel<T>::Tb(L)[cls * TSTRIDE + NSLOT] : num / c0;
+    if (L.table) x[cell] = num * Sel<T>::Tb(L)[cls * TSTRIDE + NSLOT];
+    else x[cell] = quotient(num, c0);
+}
+
+// The two bodies above for a level with coefficient arrays, with every load ahead of the arithmetic (the
+// general form's tests per neighbour leave one load in flight at a time): the same operations in the same
+// order.  `update`: Gauss-Seidel, else the residual.
+template <typename T, int ND, bool update>
+__device__ __forceinline__ void array_cell(const LvlDev& L, int i, int j, int k) {
+    const int n0 = L.n[0], n1 = ND > 1 ? L.n[1] : 1, n2 = ND > 2 ? L.n[2] : 1;
+    const long long sz = (long long) n0 * n1, cell = (long long) i + (long long) n0 * j + sz * k;
+    T* __restrict__ x = Sel<T>::x(L);
+    const T* __restrict__ A = Sel<T>::A(L) + cell;
+    const T* p = x + cell;
+    bool has[2 * ND];
+    T v[2 * ND], cf[2 * ND + 1];
+    {
+        has[0] = i > 0 || L.per[0];
+        has[1] = i < n0 - 1 || L.per[0];
+        v[0] = p[i > 0 ? -1 : has[0] ? n0 - 1 : 0];
+        v[1] = p[i < n0 - 1 ? 1 : has[1] ? 1 - n0 : 0];
+    }
+    if constexpr (ND > 1) {
+        has[2] = j > 0 || L.per[1];
+        has[3] = j < n1 - 1 || L.per[1];
+        v[2] = p[j > 0 ? -(long long) n0 : has[2] ? sz - n0 : 0];
+        v[3] = p[j < n1 - 1 ? (long long) n0 : has[3] ? n0 - sz : 0];
+    }
+    if constexpr (ND > 2) {
+        const long long all = sz * (n2 - 1);
+        has[4] = k > 0 || L.per[2];
+        has[5] = k < n2 - 1 || L.per[2];
+        v[4] = p[k > 0 ? -sz : has[4] ? all : 0];
+        v[5] = p[k < n2 - 1 ? sz : has[5] ? -all : 0];
+    }
+#pragma unroll
+    for (int q = 0; q <= 2 * ND; ++q) cf[q] = A[(long long) q * L.N];
+    const T b = Sel<T>::b(L)[cell], c = update ? (T) 0 : *p;
+    T acc = 0;
+#pragma unroll
+    for (int q = 0; q < 2 * ND; ++q) {
+        const T t = acc + cf[q + 1] * v[q];
+        acc = has[q] ? t : acc;
+    }
+    if constexpr (update) x[cell] = quotient(b - acc, cf[0]);
+    else Sel<T>::r(L)[cell] = b - (cf[0] * c + acc);
 }
 
 // damped Jacobi in two phases: 0 forms r = b - A x, 1 applies x += 0.8 r / diag
@@ -173,49 +219,57 @@ __device__ __forceinline__ T coarse_at(const LvlDev& Lc, const T* xc, int I0, in
     return xc[cell_of(Lc, I[0], I[1], I[2])];
 }
 
-// fine x += P x_coarse at fine cell f.  FAST adds a path for cell-centred fine cells whose coarse
-// neighbours are all inside the box (the same terms in the same order, sign 1); the chunked
-// float32 prolongation uses it, the tile and bottom kernels (tight on registers) do not.
-template <typename T, bool FAST = false>
+// Bi- / trilinear interpolation at fine cell f of a cell-centred level: 3/4 from the nearest coarse cell, 1/4
+// from the next one per direction.  A neighbour outside the box is the cell that its ghost rule names, its
+// sign turned where the rule turns it (an integer operation); the weights are constants (exact products), and
+// the loads precede the sum.  Inside and at the boundary alike, so that a row's end cells hold up no warp.
+__device__ __forceinline__ double turn(double v, int s) { return __hiloint2double(__double2hiint(v) ^ s, __double2loint(v)); }
+__device__ __forceinline__ float turn(float v, int s) { return __int_as_float(__float_as_int(v) ^ s); }
+template <typename T, int ND>
+__device__ __forceinline__ T prolong_cells(const LvlDev& Lc, const T* __restrict__ xc, int f0, int f1, int f2) {
+    constexpr int NZ = ND > 2 ? 2 : 1, NY = ND > 1 ? 2 : 1;
+    int idx[3][2], sgn[3][2];  // [direction][nearest, next]
+    const int f[3] = {f0, f1, f2};
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            int q = e == 0 ? f[d] >> 1 : (f[d] >> 1) + ((f[d] & 1) ? 1 : -1), s = 0;
+            const int n = Lc.n[d];
+            if (q < 0 || q >= n) {
+                const int g = q < 0 ? Lc.gh_lo[d] : Lc.gh_hi[d];
+                const int over = q < 0 ? 0 : n - 1;
+                s = g == GH_WRAP || g == GH_COPY ? 0 : (int) 0x80000000;
+                q = g == GH_WRAP ? (q < 0 ? q + n : q - n) : over;
+            }
+            idx[d][e] = q;
+            sgn[d][e] = s;
+        }
+    T v[NZ * NY * 2], acc = 0;
+#pragma unroll
+    for (int q = 0; q < NZ * NY * 2; ++q) {
+        const int e = q & 1, b = (q >> 1) & 1, a = q >> 2;
+        v[q] = turn(xc[cell_of(Lc, idx[0][e], ND > 1 ? idx[1][b] : 0, ND > 2 ? idx[2][a] : 0)], sgn[0][e] ^ (ND > 1 ? sgn[1][b] : 0) ^ (ND > 2 ? sgn[2][a] : 0));
+    }
+#pragma unroll
+    for (int q = 0; q < NZ * NY * 2; ++q)
+        acc += (q & 1 ? (T) 0.25 : (T) 0.75) * (ND > 1 ? (q & 2 ? (T) 0.25 : (T) 0.75) : (T) 1) * (ND > 2 ? (q & 4 ? (T) 0.25 : (T) 0.75) : (T) 1) * v[q];
+    return acc;
+}
+
+// fine x += P x_coarse at fine cell f
+template <typename T>
 __device__ __forceinline__ T prolong_acc(const LvlDev* __restrict__ Ls, const LvlDev& Lf, int f0, int f1, int f2) {
     const LvlDev& Lc = Ls[Lf.coarse];
     const T* xc = Sel<T>::x(Lc);
-    const int f[3] = {f0, f1, f2};
     T acc = 0;
     if (!Lc.node) {
-        // bilinear / trilinear on cell centres: 3/4 nearest coarse cell, 1/4 the next one
-        int I[3], J[3];
-        for (int d = 0; d < 3; ++d) {
-            I[d] = f[d] >> 1;
-            J[d] = (f[d] & 1) ? I[d] + 1 : I[d] - 1;
-        }
-        const int nz = Lc.ndim > 2 ? 2 : 1, ny = Lc.ndim > 1 ? 2 : 1;
-        bool inside = FAST;
-        for (int d = 0; FAST && d < Lc.ndim; ++d) inside = inside && I[d] >= 0 && I[d] < Lc.n[d] && J[d] >= 0 && J[d] < Lc.n[d];
-        if (FAST && inside) {
-            // every coarse neighbour inside the box: the terms below with sign 1, in their order
-            for (int a = 0; a < nz; ++a)
-                for (int bb = 0; bb < ny; ++bb)
-                    for (int e = 0; e < 2; ++e) {
-                        const T w = (e ? (T) 0.25 : (T) 0.75) * (Lc.ndim > 1 ? (bb ? (T) 0.25 : (T) 0.75) : (T) 1) *
-                                    (Lc.ndim > 2 ? (a ? (T) 0.25 : (T) 0.75) : (T) 1);
-                        const T v = xc[cell_of(Lc, e ? J[0] : I[0], Lc.ndim > 1 ? (bb ? J[1] : I[1]) : 0, Lc.ndim > 2 ? (a ? J[2] : I[2]) : 0)];
-                        acc += w * (T) 1 * v;
-                    }
-            return acc;
-        }
-        for (int a = 0; a < nz; ++a)
-            for (int bb = 0; bb < ny; ++bb)
-                for (int e = 0; e < 2; ++e) {
-                    const T w = (e ? (T) 0.25 : (T) 0.75) * (Lc.ndim > 1 ? (bb ? (T) 0.25 : (T) 0.75) : (T) 1) *
-                                (Lc.ndim > 2 ? (a ? (T) 0.25 : (T) 0.75) : (T) 1);
-                    T s;
-                    const T v = coarse_at<T>(Lc, xc, e ? J[0] : I[0], Lc.ndim > 1 ? (bb ? J[1] : I[1]) : 0, Lc.ndim > 2 ? (a ? J[2] : I[2]) : 0, s);
-                    acc += w * s * v;
-                }
+        if (Lc.ndim == 3) return prolong_cells<T, 3>(Lc, xc, f0, f1, f2);
+        if (Lc.ndim == 2) return prolong_cells<T, 2>(Lc, xc, f0, f1, f2);
+        return prolong_cells<T, 1>(Lc, xc, f0, f1, f2);
     } else {
         // linear interpolation on nodes: absolute fine node g <-> coarse node g/2
-        const int g[3] = {Lf.lo[0] + f[0], Lf.lo[1] + f[1], Lf.lo[2] + f[2]};
+        const int g[3] = {Lf.lo[0] + f0, Lf.lo[1] + f1, Lf.lo[2] + f2};
         int c0[3], c1[3];
         T w0[3], w1[3];
         for (int d = 0; d < 3; ++d) {
@@ -246,9 +300,9 @@ __device__ __forceinline__ T prolong_acc(const LvlDev* __restrict__ Ls, const Lv
     return acc;
 }
 
-template <typename T, bool FAST = false>
+template <typename T>
 __device__ __forceinline__ void cell_prolong(const LvlDev* __restrict__ Ls, const LvlDev& Lf, int f0, int f1, int f2) {
-    const T acc = prolong_acc<T, FAST>(Ls, Lf, f0, f1, f2);
+    const T acc = prolong_acc<T>(Ls, Lf, f0, f1, f2);
     Sel<T>::x(Lf)[cell_of(Lf, f0, f1, f2)] += acc;
 }
 

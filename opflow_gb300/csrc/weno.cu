@@ -22,6 +22,7 @@
 // 16384 lines of 4096 cells 44.2 -> 35.2 ms.
 // FAST mode (not bit-identical) contracts the arithmetic and forms the three nonlinear weights with one
 // reciprocal.
+#include "f64div.h"
 #include "stencil.h"
 
 #include <cmath>
@@ -47,7 +48,6 @@ struct WenoParams {
 
 // The rare sides of the divisions below, apart: of a branch within the code the compiler issues both sides
 // under predicates, and a float64 operation that is predicated off takes its time all the same.
-static __device__ __noinline__ double weno_div(double a, double b) { return __ddiv_rn(a, b); }
 static __device__ __noinline__ double weno_mul(double a, double b) { return __dmul_rn(a, b); }
 
 // Whether x is neither zero nor, with a wide margin, in the normal range: the steps below are not exact there.
@@ -58,16 +58,6 @@ __device__ __forceinline__ bool out_of_range(double x) {
 
 // correctly rounded x / c for the c whose reciprocal is ch + cl, x in range
 __device__ __forceinline__ double div_const(double x, double ch, double cl) { return __fma_rn(x, ch, __dmul_rn(x, cl)); }
-
-// 1/x for x in the normal range: the hardware's approximate reciprocal refined by the cubic Newton step
-// y = r + r*(e + e^2), e = 1 - x*r (Newton-Raphson iteration for 1/x with the second-order term; the
-// relative error goes from eps to about eps^3).
-__device__ __forceinline__ double recip_fast(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = __fma_rn(-x, r, 1.0);
-    return __fma_rn(__fma_rn(e, e, e), r, r);
-}
 
 // a / b, correctly rounded, given y = 1/b to within an ulp (recip_fast): q = a y, the exact remainder
 // r = a - q b, and q + r y (the division steps of Markstein, IBM J. Res. Dev. 34 (1990)).  q is off a / b
@@ -92,7 +82,7 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
     const int k = (int) (rb >> 52) - (int) (T >> 52);
     const unsigned long long mr = ((rb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << (k & 3), mb = 3 * ((bb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull);
     bad |= (k == 1 || k == 2) && mr - mb + 256 <= 512;
-    if (bad) v = weno_div(a, b);
+    if (bad) v = div_apart(a, b);
     return v;
 }
 
@@ -123,9 +113,9 @@ __device__ __forceinline__ double dh_of(double a, const WenoParams& P) {
         if (!zero && ((unsigned) (e - 1) >= 2046u || (unsigned) (e + P.h_shift - 1) >= 2046u)) r = weno_mul(a, P.inv_h);
         return r;
     }
-    if (!P.h_two) return weno_div(a, P.h);
+    if (!P.h_two) return div_apart(a, P.h);
     double r = div_const(a, P.inv_h, P.h_cl);
-    if (out_of_range(a) || (P.h_guard && lo == P.bad_lo && (hi & 0xFFFFF) == P.bad_hi)) r = weno_div(a, P.h);
+    if (out_of_range(a) || (P.h_guard && lo == P.bad_lo && (hi & 0xFFFFF) == P.bad_hi)) r = div_apart(a, P.h);
     return r;
 }
 
@@ -141,10 +131,10 @@ __device__ __forceinline__ DiffTerms diff_terms(double lo, double hi, const Weno
         t.D76 = div_const(__dmul_rn(7., t.D), P.r6, P.cl6);
         t.D116 = div_const(__dmul_rn(11., t.D), P.r6, P.cl6);
         if (out_of_range(t.D)) {
-            t.D3 = weno_div(t.D, 3.);
-            t.D56 = weno_div(weno_mul(5., t.D), 6.);
-            t.D76 = weno_div(weno_mul(7., t.D), 6.);
-            t.D116 = weno_div(weno_mul(11., t.D), 6.);
+            t.D3 = div_apart(t.D, 3.);
+            t.D56 = div_apart(weno_mul(5., t.D), 6.);
+            t.D76 = div_apart(weno_mul(7., t.D), 6.);
+            t.D116 = div_apart(weno_mul(11., t.D), 6.);
         }
         t.M3 = __dmul_rn(3., t.D);
     }

@@ -15,7 +15,7 @@ BC = {"neum": capi.BC_NEUM, "dirc": capi.BC_DIRC, "per": capi.BC_PERIODIC}
 TOL = 1e-9
 
 
-def _solve(ctx, n, bc, array, prec, scale=1.0, guess=True, tol=TOL):
+def _solve(ctx, n, bc, array, prec, scale=1.0, guess=True, tol=TOL, A=1.0):
     D = len(n)
     mesh = cm.mesh_uniform([m + 1 for m in n])
     fd = cm.field_desc(D, capi.CENTER, [(BC[bc], BC[bc])] * D, ext=1)
@@ -24,14 +24,14 @@ def _solve(ctx, n, bc, array, prec, scale=1.0, guess=True, tol=TOL):
     rng = np.random.default_rng(sum(n))
     for x, v in ((f, rng.standard_normal), (p, rng.standard_normal), (c, lambda s: 1.0 + rng.random(s))):
         a = x.download()
-        a[sl] = v(a[sl].shape) * (1.0 if x is c else scale)
+        a[sl] = v(a[sl].shape) * (A if x is c else scale)
         x.upload(a)
     d2 = [api.d2x, api.d2y, api.d2z][:D]
 
     def op(e):
         t = c * e if array else 1.0 * e
         for d, m in zip(d2, n):
-            t = t - 0.2 / m ** 2 * d(e)
+            t = t - A * 0.2 / m ** 2 * d(e)
         return t
     par = api.StructSolverParams(tol=tol, maxIter=60, precision=prec, zeroGuess=not guess)
     st = api.Solve(lambda e: api.Eq(op(e), f), p, par)
@@ -67,3 +67,13 @@ def test_residuals_that_are_subnormal_in_float32(ctx, n):
     # values around 2^-130 in float32: 19 bits and fewer, still a preconditioner
     st, res, _ = _solve(ctx, n, "dirc", False, "mixed", scale=2.0 ** -130, guess=False, tol=1e-2)
     assert st.converged and res <= 1.001e-2, (st, res)
+
+
+@pytest.mark.parametrize("n", [[130], [70, 50], [40, 33, 19]])
+@pytest.mark.parametrize("k", [-900, 900])
+def test_array_levels_scaled_to_the_ends_of_the_range(ctx, n, k):
+    # the diagonal's exponent leaves the range of the six-operation quotient: IEEE divisions, the same bits
+    want = _solve(ctx, n, "dirc", True, "fp64", guess=False)
+    got = _solve(ctx, n, "dirc", True, "fp64", guess=False, A=2.0 ** k)
+    assert got[0].niter == want[0].niter
+    assert np.array_equal(got[2], want[2] * 2.0 ** -k)
