@@ -6,6 +6,7 @@
 // program can reach; "absent" and "zero" coincide there, which changes no value.
 #include "assemble.h"
 #include "pointwise.h"
+#include "tape.h"
 
 #include <cmath>
 #include <map>
@@ -583,6 +584,95 @@ static void plain_rhs(const std::vector<PInstr>& prog, AsmPlan* plan) {
     for (int d = 0; d < 3; ++d) plan->rhs_off[d] = r.in.off[d];
 }
 
+// The inner cells' coefficients and right-hand side as a scalar program: there every leaf of the unknown is one
+// coefficient 1 and no bias, so a pad's entries are values or absent, and only the present ones are formed
+// (the reference's StencilPad holds no others either).  coef: with the coefficients, else the right-hand side
+// alone.
+static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
+    const AsmParams& P = plan.P;
+    struct Pad { std::map<int, int> c; int b = -1; };  // entry -> value, bias value (-1: none)
+    std::vector<Pad> pads;
+    std::vector<int> nums;
+    auto num = [&] { const int v = nums.back(); nums.pop_back(); return v; };
+    for (const PInstr& in : plan.prog) {
+        switch (in.op) {
+            case Q_LOADS: nums.push_back(T->load(in.slot, P.leaves[in.slot], in.off)); break;
+            case Q_LOADU: {
+                Pad p;
+                int k = -1;
+                for (int q = 0; q < P.nk; ++q)
+                    if (P.K[q][0] == in.off[0] && P.K[q][1] == in.off[1] && P.K[q][2] == in.off[2]) k = q;
+                if (k < 0) return false;
+                if (coef) p.c[k] = T->cst(1.0);
+                pads.push_back(p);
+                break;
+            }
+            case Q_CONST: nums.push_back(T->cst(in.v)); break;
+            case Q_DX: nums.push_back(T->pos(T_DX, in.slot, in.off[0])); break;
+            case Q_X: nums.push_back(T->pos(T_X, in.slot, in.off[0])); break;
+            case Q_NEG:
+                if (in.ta) {
+                    for (auto& e : pads.back().c) e.second = T->neg(e.second);
+                    if (pads.back().b >= 0) pads.back().b = T->neg(pads.back().b);
+                } else nums.back() = T->neg(nums.back());
+                break;
+            case Q_NOT: nums.back() = T->node(T_NOT, 0, nums.back()); break;
+            case Q_F1: nums.back() = T->node(T_F1, in.slot, nums.back()); break;
+            case Q_F2: {
+                const int b = num(), a = num();
+                nums.push_back(T->node(T_F2, in.slot, a, b));
+                break;
+            }
+            case Q_SEL: {
+                const int b = num(), a = num(), c = num();
+                nums.push_back(T->node(T_SEL, 0, c, a, b));
+                break;
+            }
+            case Q_GT: case Q_GE: case Q_LT: case Q_LE: case Q_NE: case Q_AND: case Q_OR: {
+                static const int cmp[] = {T_GT, T_GE, T_LT, T_LE, T_NE, T_AND, T_OR};
+                const int b = num(), a = num();
+                nums.push_back(T->bin(cmp[in.op - Q_GT], a, b));
+                break;
+            }
+            default: {
+                static const int ops[] = {T_ADD, T_SUB, T_MUL, T_DIV};
+                const int op = ops[in.op - Q_ADD];
+                if (!in.ta && !in.tb) {
+                    const int b = num(), a = num();
+                    nums.push_back(T->bin(op, a, b));
+                    break;
+                }
+                Pad B, A;
+                if (in.tb) { B = pads.back(); pads.pop_back(); } else B.b = num();
+                if (in.ta) { A = pads.back(); pads.pop_back(); } else A.b = num();
+                if (op == T_ADD || op == T_SUB) {
+                    auto both = [&](int a, int b) { return a < 0 ? (b < 0 ? -1 : op == T_ADD ? b : T->neg(b)) : b < 0 ? a : T->bin(op, a, b); };
+                    for (auto& e : B.c) {
+                        auto it = A.c.find(e.first);
+                        A.c[e.first] = both(it == A.c.end() ? -1 : it->second, e.second);
+                    }
+                    A.b = both(A.b, B.b);
+                } else {
+                    // a product with a number, or pad / num = pad * (1. / num)
+                    const int s = op == T_DIV ? T->bin(T_DIV, T->cst(1.0), B.b) : in.ta ? B.b : A.b;
+                    if (!in.ta) A = B;
+                    for (auto& e : A.c) e.second = T->bin(T_MUL, e.second, s);
+                    if (A.b >= 0) A.b = T->bin(T_MUL, A.b, s);
+                }
+                pads.push_back(A);
+            }
+        }
+    }
+    const Pad& r = pads.back();
+    if (coef)
+        for (int q = 0; q < P.nk; ++q) T->out(T_COEF, q, r.c.count(q) ? r.c.at(q) : T->cst(0.0));
+    T->out(T_RHS, 0, r.b >= 0 ? T->neg(r.b) : T->cst(0.0));
+    return true;
+}
+
+// Cells of the inner box from which its program is run apart from the shell's (below that one launch for both).
+constexpr long long ASM_TAPE_CELLS = 4096;
+
 // ======================================================================== host structural evaluation
 // Key order of the middle cell's StencilPad (fake_map insertion order): the recursion of the
 // reference with only the keys tracked.
@@ -779,8 +869,9 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
     int* err = (int*) ctx->scratch;
     cudaMemsetAsync(err, 0, sizeof(int), ctx->stream);
     cudaMemcpyAsync(dprog, plan->prog.data(), plan->prog.size() * sizeof(PInstr), cudaMemcpyHostToDevice, ctx->stream);
-    // the right-hand side alone: inner cells as one plain field where they are, the shell around them by
-    // the program (256^3 cells of f == d2x(p) + d2y(p) + d2z(p): 3.39 ms by the program, about 50 us here)
+    // Inner cells: one plain field (the right-hand side alone, where they are; 256^3 cells of
+    // f == d2x(p) + d2y(p) + d2z(p): 3.39 ms by the general program, 78 us so), else their scalar program
+    // (the flux form's coefficients at 192^3: 8.5 -> 1.5 ms and the shell's 0.4); the shell around them by the general program.
     AsmCells cells;
     auto add = [&](const Box& b) {
         if (b.empty()) return;
@@ -790,11 +881,39 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
     };
     cells.start[0] = 0;
     const Box &all = plan->P.box, &in = plan->inner;
-    if (!coef && plan->rhs_plain && !plan->P.pin && !in.empty()) {
+    // a pinned unknown among the inner cells' leaves has no coefficient there
+    bool pinned = false;
+    for (const PInstr& q : plan->prog) {
+        bool hit = plan->P.pin != 0 && q.op == Q_LOADU;
+        for (int d = 0; d < plan->P.ndim; ++d) hit = hit && plan->P.pin_index[d] - q.off[d] >= in.lo[d] && plan->P.pin_index[d] - q.off[d] < in.hi[d];
+        pinned |= hit;
+    }
+    const bool plain = !coef && plan->rhs_plain && !plan->P.pin && !in.empty();
+    Tape tape;
+    bool taped = false;
+    if (!plain && !pinned && in.count() >= ASM_TAPE_CELLS) taped = inner_tape(*plan, coef != nullptr, &tape) && tape.finish(in, in.count() >= 32768);
+    int rc = OPFLOW_OK;
+    if (plain) {
         const int nx = in.hi[0] - in.lo[0], rows = (in.hi[1] - in.lo[1]) * (in.hi[2] - in.lo[2]);
         plain_rhs_kernel<<<dim3((nx + 255) / 256, std::min(rows, 65535)), 256, 0, ctx->stream>>>(plan->P.leaves[plan->rhs_slot], all, in, plan->rhs_off[0],
                                                                                             plan->rhs_off[1], plan->rhs_off[2], plan->rhs_sign, rhs);
         OPG_LAUNCHED();
+    } else if (taped) {
+        TapeArgs A{};
+        for (int s = 0; s < 8; ++s) A.leaves[s] = plan->P.leaves[s];
+        for (int d = 0; d < 3; ++d) {
+            A.x[d] = plan->P.mx[d];
+            A.dx[d] = plan->P.mdx[d];
+            A.es[d] = plan->P.es[d];
+        }
+        A.box = A.tab_box = in;
+        A.rows = all;
+        A.coef = coef;
+        A.rhs = rhs;
+        rc = tape.prepare(ctx, A);
+        if (rc == OPFLOW_OK) rc = tape.run(ctx, A);
+    }
+    if (plain || taped) {
         Box rest = all;
         for (int d = 2; d >= 0; --d) {
             Box lo = rest, hi = rest;
@@ -814,11 +933,12 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
         else assemble_kernel<true><<<(int) blocks, 128, 0, ctx->stream>>>(dprog, (int) plan->prog.size(), plan->P, cells, coef, rhs, err);
         OPG_LAUNCHED();
     }
-    int rc = check_launch("assemble_kernel");
+    if (rc == OPFLOW_OK) rc = check_launch("assemble_kernel");
     int herr = 0;
     cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     dev_free(ctx, dprog);
+    tape.release(ctx);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(OPFLOW_E_CUDA, "assembly failed: %s", cudaGetErrorString(e));
     if (herr) return fail(OPFLOW_E_RANGE, "a folded unknown leaf left the stencil offset set or the logical range");

@@ -8,11 +8,13 @@
 //   2. In OPFLOW_EVAL_FAST mode, a tree that is a linear constant-coefficient stencil of one field goes
 //      to a fixed-point kernel (exact 64-bit integer sums, one product per weight group, one rounding
 //      back to float64 per point) that runs on the integer pipes instead of GB300's narrow FP64 pipe.
-//   3. Everything else runs in a generic interpreter kernel over a postfix program expanded from the
-//      tree, again in the reference's operation order.
+//   3. Everything else runs as a scalar program over the cells (tape.h), formed from a postfix program
+//      expanded from the tree, with the reference's operations; what holds a WENO operator or needs too many
+//      values at once, and the items of a batch, as that postfix program itself (interp_cell).
 #include "internal.h"
 #include "stencil_exact.h"
 #include "pointwise.h"
+#include "tape.h"
 
 #include <algorithm>
 #include <array>
@@ -761,6 +763,8 @@ struct Plan {
     bool aliased = false;
     Box box;
     std::vector<Instr> prog;
+    bool taped = false;  // PLAN_INTERP: `tape` runs it, else the stack program (dprog)
+    Tape tape;
     Instr* dprog = nullptr;
     LeafViews leaves{};
     MeshPtrs mesh{};
@@ -1055,15 +1059,78 @@ static int build_plan(opflow_ctx ctx, opflow_field dst, int arith, const opflow_
             }
         }
     }
-    if (plan->kind == PLAN_INTERP && !plan->prog.empty()) {
-        OPG_CUDA(cudaMalloc(&plan->dprog, plan->prog.size() * sizeof(Instr)));
-        OPG_CUDA(cudaMemcpyAsync(plan->dprog, plan->prog.data(), plan->prog.size() * sizeof(Instr), cudaMemcpyHostToDevice, ctx->stream));
-    }
     return OPFLOW_OK;
 }
 
-static void free_plan(Plan* p) {
-    if (p->dprog) cudaFree(p->dprog);
+// The stack program as a scalar program over the cells; false where it holds what that has no form for.
+static bool tape_of(const std::vector<Instr>& prog, const LeafViews& leaves, Tape* T) {
+    std::vector<int> st;
+    auto pop = [&] { const int v = st.back(); st.pop_back(); return v; };
+    for (const Instr& in : prog) {
+        switch (in.op) {
+            case P_LOAD: st.push_back(T->load(in.slot, leaves.v[in.slot], in.off)); break;
+            case P_CONST: st.push_back(T->cst(in.v)); break;
+            case P_DX: st.push_back(T->pos(T_DX, in.slot, in.off[0])); break;
+            case P_X: st.push_back(T->pos(T_X, in.slot, in.off[0])); break;
+            case P_NEG: st.back() = T->neg(st.back()); break;
+            case P_NOT: st.back() = T->node(T_NOT, 0, st.back()); break;
+            case P_F1: st.back() = T->node(T_F1, in.slot, st.back()); break;
+            case P_LIM: st.back() = T->node(T_LIM, in.slot, st.back()); break;
+            case P_SEL: {
+                const int b = pop(), a = pop(), c = pop();
+                st.push_back(T->node(T_SEL, 0, c, a, b));
+                break;
+            }
+            case P_F2: {
+                const int b = pop(), a = pop();
+                st.push_back(T->node(T_F2, in.slot, a, b));
+                break;
+            }
+            case P_WENO: return false;
+            default: {
+                static const int ops[] = {T_ADD, T_SUB, T_MUL, T_DIV}, cmp[] = {T_GT, T_GE, T_LT, T_LE, T_NE, T_AND, T_OR};
+                const int b = pop(), a = pop();
+                st.push_back(T->bin(in.op <= P_DIV ? ops[in.op - P_ADD] : cmp[in.op - P_GT], a, b));
+            }
+        }
+    }
+    T->out(T_OUT, 0, st.back());
+    return true;
+}
+
+static TapeArgs tape_args(const Plan& plan, const FieldView& out, const FieldView& cur, int arith) {
+    TapeArgs A{};
+    for (int s = 0; s < plan.leaves.n; ++s) A.leaves[s] = plan.leaves.v[s];
+    for (int d = 0; d < 3; ++d) {
+        A.x[d] = plan.mesh.x[d];
+        A.dx[d] = plan.mesh.dx[d];
+        A.es[d] = plan.mesh.es[d];
+    }
+    A.box = A.tab_box = plan.box;
+    A.out = out;
+    A.cur = cur;
+    A.arith = arith;
+    return A;
+}
+
+// the device side of an interpreted plan
+static int plan_device(opflow_ctx ctx, opflow_field dst, const opflow_field* leaves, int arith, Plan* plan) {
+    if (plan->kind != PLAN_INTERP || plan->prog.empty() || plan->box.empty()) return OPFLOW_OK;
+    for (int s = 0; s < plan->leaves.n; ++s) plan->leaves.v[s] = leaves[s]->view();
+    // (tables of one direction's values: a launch per direction, worth it from about 2^15 cells)
+    if (tape_of(plan->prog, plan->leaves, &plan->tape) && plan->tape.finish(plan->box, plan->box.count() >= 32768)) {
+        plan->taped = true;
+        return plan->tape.prepare(ctx, tape_args(*plan, dst->view(), dst->view(), arith));
+    }
+    plan->dprog = (Instr*) dev_alloc(ctx, plan->prog.size() * sizeof(Instr));
+    if (!plan->dprog) return fail(OPFLOW_E_NOMEM, "expression program");
+    OPG_CUDA(cudaMemcpyAsync(plan->dprog, plan->prog.data(), plan->prog.size() * sizeof(Instr), cudaMemcpyHostToDevice, ctx->stream));
+    return OPFLOW_OK;
+}
+
+static void free_plan(opflow_ctx ctx, Plan* p) {
+    p->tape.release(ctx);
+    if (p->dprog) dev_free(ctx, p->dprog);
     p->dprog = nullptr;
 }
 
@@ -1208,6 +1275,10 @@ static int run_plan(opflow_ctx ctx, opflow_field dst, int arith, const opflow_fi
                 break;
             }
             default: {
+                if (plan->taped) {
+                    OPG_TRY(plan->tape.run(ctx, tape_args(*plan, out, cur, arith)));
+                    break;
+                }
                 const int g = grid_for(ctx, total, 128);
                 interp_kernel<<<g, 128, 0, ctx->stream>>>(plan->dprog, (int) plan->prog.size(), plan->leaves, plan->mesh, plan->box, out, cur, arith);
                 OPG_LAUNCHED();
@@ -1232,11 +1303,12 @@ int opflow_assign_repeat(opflow_ctx ctx, opflow_field dst, int arith, const opfl
     if (steps == 0) return OPFLOW_OK;
     Plan plan;
     int rc = build_plan(ctx, dst, arith, nodes, n_nodes, leaves, n_leaves, mode, &plan);
-    if (rc) { free_plan(&plan); return rc; }
+    if (rc == OPFLOW_OK) rc = plan_device(ctx, dst, leaves, arith, &plan);
+    if (rc) { free_plan(ctx, &plan); return rc; }
     unsigned long long* maxslots = nullptr;
     if (plan.kind == PLAN_FAST || plan.kind == PLAN_AXIS_FAST) {
         rc = ensure_scratch(ctx, 256);
-        if (rc) { free_plan(&plan); return rc; }
+        if (rc) { free_plan(ctx, &plan); return rc; }
         maxslots = (unsigned long long*) ctx->scratch;
         cudaMemsetAsync(maxslots, 0, 3 * sizeof(unsigned long long), ctx->stream);
         // the source's readable values bound the fixed-point scale of the first step
@@ -1246,7 +1318,7 @@ int opflow_assign_repeat(opflow_ctx ctx, opflow_field dst, int arith, const opfl
         maxabs_kernel<<<grid_for(ctx, all.count(), 256), 256, 0, ctx->stream>>>(src->view(), all, maxslots);
         OPG_LAUNCHED();
         rc = check_launch("maxabs_kernel");
-        if (rc) { free_plan(&plan); return rc; }
+        if (rc) { free_plan(ctx, &plan); return rc; }
     }
     if (resident_eligible(plan, dst, leaves, steps)) {
         // fixed point kept in the field's buffers between the steps of the run (axis3d_fxres_kernel)
@@ -1255,7 +1327,7 @@ int opflow_assign_repeat(opflow_ctx ctx, opflow_field dst, int arith, const opfl
         for (int s = 0; s < steps && rc == OPFLOW_OK; ++s) rc = run_plan(ctx, dst, arith, leaves, &plan, maxslots, s);
     }
     if (rc == OPFLOW_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = fail(OPFLOW_E_CUDA, "assign failed: %s", cudaGetErrorString(cudaGetLastError()));
-    free_plan(&plan);
+    free_plan(ctx, &plan);
     return rc;
 }
 
@@ -1287,7 +1359,6 @@ int opflow_assign_batch(opflow_ctx ctx, int n, const opflow_field* dsts, const i
     for (int i = 0; i < n && rc == OPFLOW_OK; ++i) {
         // exact mode for every item: the FTCS cell where the expression has that shape, else the interpreter
         rc = build_plan(ctx, dsts[i], arith[i], nodes[i], n_nodes[i], leaves[i], n_leaves[i], OPFLOW_EVAL_EXACT, &plans[i]);
-        free_plan(&plans[i]);
         if (rc == OPFLOW_OK && plans[i].aliased) rc = ensure_back(dsts[i]);
         prog_at[i] = (int) progs.size();
         progs.insert(progs.end(), plans[i].prog.begin(), plans[i].prog.end());

@@ -28,6 +28,46 @@ __device__ __forceinline__ double quotient(double a, double b) {
     if ((unsigned) (eb - 200) > 1600u || ((unsigned) (ea - 200) > 1600u && ((__double2hiint(a) & 0x7FFFFFFF) | __double2loint(a)) != 0)) v = div_apart(a, b);
     return v;
 }
+// a / b, correctly rounded, given y = 1/b to within an ulp (recip_fast): q = a y, the remainder r = a - q b, and
+// q + r y (the division steps of Markstein, as above).  q is off a / b by less than 1.6 ulps of q and y by 2^-52
+// of 1/b, so q + r y is off a / b by less than 2^-51 ulp before its rounding; it is rounded to a / b's neighbour
+// unless a / b lies that near the middle of two numbers.  That is looked for on the bits (integer operations,
+// which cost next to nothing here): |r| near ulp(q) b / 2 or 3 ulp(q) b / 2, or q next to a power of two (below
+// it the numbers are denser); then, and where an exponent is near the ends of the range, the lanes concerned
+// divide.  SIGNED: operands of either sign and zero numerators (else positive ones, or the division apart).
+template <bool SIGNED>
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+    constexpr unsigned long long MAG = 0x7FFFFFFFFFFFFFFFull, FRAC = 0xFFFFFFFFFFFFFull, ONE = 0x10000000000000ull;
+    const double q = __dmul_rn(a, y);
+    const double r = __fma_rn(-q, b, a);
+    double v = __fma_rn(r, y, q);
+    unsigned long long ab = (unsigned long long) __double_as_longlong(a), bb = (unsigned long long) __double_as_longlong(b),
+                       qb = (unsigned long long) __double_as_longlong(q);
+    const unsigned long long rb = (unsigned long long) __double_as_longlong(r) & MAG;
+    if (SIGNED) {
+        ab &= MAG;
+        bb &= MAG;
+        qb &= MAG;
+    }
+    const unsigned ea = (unsigned) (ab >> 52), eb = (unsigned) (bb >> 52), eq = (unsigned) (qb >> 52);
+    bool bad = ea - 200u > 1600u || eq - 200u > 1600u;
+    bad |= (qb & FRAC) < 3;
+    // T = ulp(q) b / 2
+    const unsigned long long T = bb + ((unsigned long long) eq << 52) - ((unsigned long long) (1023 + 53) << 52);
+    bad |= rb - T + 64 <= 128;
+    // |r| against 3 T: significands 2^k m(r) and 3 m(b), k the difference of the exponents
+    const int k = (int) (rb >> 52) - (int) (T >> 52);
+    const unsigned long long mr = ((rb & FRAC) | ONE) << (k & 3), mb = 3 * ((bb & FRAC) | ONE);
+    bad |= (k == 1 || k == 2) && mr - mb + 256 <= 512;
+    if (SIGNED && ab == 0) {
+        bad = false;
+        v = q;  // (a zero of the right sign)
+    }
+    bad |= eb - 200u > 1600u;
+    if (bad) v = div_apart(a, b);
+    return v;
+}
+
 __device__ __forceinline__ float quotient(float a, float b) { return a / b; }
 
 }  // namespace opg

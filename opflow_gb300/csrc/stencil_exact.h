@@ -19,6 +19,7 @@
 // 19 cycles at best: 16.2 us), 301 x 257 x 333 (one power of two) 2074 -> 1010 us, 64 grids of 4.35 M points
 // 226 -> 158 us.
 #pragma once
+#include "f64div.h"
 #include "stencil.h"
 
 namespace opg {
@@ -41,7 +42,6 @@ inline int exact_mode(const AxisParams& P) {
 // sides under predicates, and a float64 operation that is predicated off takes its 16 cycles of the pipe
 // all the same (measured).
 static __device__ __noinline__ double mul_apart(double x, double y) { return __dmul_rn(x, y); }
-static __device__ __noinline__ double div_apart(double x, double y) { return __ddiv_rn(x, y); }
 
 // correctly rounded x / h[D], called by whole warps
 template <int PM, int D>

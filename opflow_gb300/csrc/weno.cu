@@ -59,33 +59,6 @@ __device__ __forceinline__ bool out_of_range(double x) {
 // correctly rounded x / c for the c whose reciprocal is ch + cl, x in range
 __device__ __forceinline__ double div_const(double x, double ch, double cl) { return __fma_rn(x, ch, __dmul_rn(x, cl)); }
 
-// a / b, correctly rounded, given y = 1/b to within an ulp (recip_fast): q = a y, the exact remainder
-// r = a - q b, and q + r y (the division steps of Markstein, IBM J. Res. Dev. 34 (1990)).  q is off a / b
-// by less than 1.5 ulps of q and y by 2^-52 of 1/b, so q + r y is off a / b by less than 2^-51 ulp before its
-// rounding; it is rounded to a / b's neighbour unless a / b lies that near the middle of two numbers.  That
-// is looked for on the bits (integer operations): |r| near ulp(q) b / 2 or 3 ulp(q) b / 2, or q next to a
-// power of two (below it the numbers are denser); then, and where an exponent is near the ends of the
-// range, the warp's lanes concerned divide.
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-    const double q = __dmul_rn(a, y);
-    const double r = __fma_rn(-q, b, a);
-    double v = __fma_rn(r, y, q);
-    const unsigned long long ab = (unsigned long long) __double_as_longlong(a), bb = (unsigned long long) __double_as_longlong(b),
-                             qb = (unsigned long long) __double_as_longlong(q), rb = (unsigned long long) __double_as_longlong(r) & 0x7FFFFFFFFFFFFFFFull;
-    const unsigned ea = (unsigned) (ab >> 52), eb = (unsigned) (bb >> 52), eq = (unsigned) (qb >> 52);  // (a, b >= 0: a sign bit fails the range test)
-    bool bad = ea - 200u > 1600u || eb - 200u > 1600u || eq - 200u > 1600u;
-    bad |= (qb & 0xFFFFFFFFFFFFFull) < 3;
-    // T = ulp(q) b / 2
-    const unsigned long long T = bb + ((unsigned long long) eq << 52) - ((unsigned long long) (1023 + 53) << 52);
-    bad |= rb - T + 64 <= 128;
-    // |r| against 3 T: significands 2^k m(r) and 3 m(b), k the difference of the exponents
-    const int k = (int) (rb >> 52) - (int) (T >> 52);
-    const unsigned long long mr = ((rb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << (k & 3), mb = 3 * ((bb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull);
-    bad |= (k == 1 || k == 2) && mr - mb + 256 <= 512;
-    if (bad) v = div_apart(a, b);
-    return v;
-}
-
 // ---- per-point arithmetic, with the terms that neighbouring points share computed once ----------------
 // A thread evaluates K consecutive points of a line.  For Downwind the point i reads the six values
 // g[p..p+5] = u[i-3..i+2] (p = i - i0); for Upwind the mirrored values u[i+3..i-2] (the line read
@@ -171,11 +144,11 @@ __device__ __forceinline__ double weno_point(const DiffTerms& X0, const DiffTerm
         const double s3 = __fma_rn(0.25, __dmul_rn(t2, t2), p2);
         const double eps = __dadd_rn(__dmul_rn(1e-6, mx), 1e-99);
         double q;
-        q = __dadd_rn(s1, eps); q = __dmul_rn(q, q); const double a1 = div_rn(.1, q, recip_fast(q));
-        q = __dadd_rn(s2, eps); q = __dmul_rn(q, q); const double a2 = div_rn(.6, q, recip_fast(q));
-        q = __dadd_rn(s3, eps); q = __dmul_rn(q, q); const double a3 = div_rn(.3, q, recip_fast(q));
+        q = __dadd_rn(s1, eps); q = __dmul_rn(q, q); const double a1 = div_rn<false>(.1, q, recip_fast(q));
+        q = __dadd_rn(s2, eps); q = __dmul_rn(q, q); const double a2 = div_rn<false>(.6, q, recip_fast(q));
+        q = __dadd_rn(s3, eps); q = __dmul_rn(q, q); const double a3 = div_rn<false>(.3, q, recip_fast(q));
         const double sum = __dadd_rn(__dadd_rn(a1, a2), a3), y = recip_fast(sum);
-        const double w1 = div_rn(a1, sum, y), w2 = div_rn(a2, sum, y), w3 = div_rn(a3, sum, y);
+        const double w1 = div_rn<false>(a1, sum, y), w2 = div_rn<false>(a2, sum, y), w3 = div_rn<false>(a3, sum, y);
         return __dadd_rn(__dadd_rn(__dmul_rn(w1, ddx1), __dmul_rn(w2, ddx2)), __dmul_rn(w3, ddx3));
     } else {
         // The same quantities with contracted arithmetic, in the scaled units above, and one reciprocal:
