@@ -96,9 +96,12 @@ __global__ void map_slots(const double* coef, long long N, const int* kslot, int
 __global__ void to_f32(const double* a, float* b, long long n) {
     for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < n; t += (long long) gridDim.x * blockDim.x) b[t] = (float) a[t];
 }
-// compare every cell's coefficients with its class representative
-__global__ void class_check(const double* A, long long N, int n0, int n1, int n2, int ndim, const double* tab, int* bad) {
-    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < N; t += (long long) gridDim.x * blockDim.x) {
+// compare every cell's coefficients with its class representative (the loads ahead of the comparisons: bound by
+// the bytes; 192^3 401 -> 20 us against one slot at a time)
+__global__ void __launch_bounds__(256) class_check(const double* __restrict__ A, long long N, int n0, int n1, int n2, int ndim, const double* __restrict__ tab,
+                                                   int* bad) {
+    bool differs = false;
+    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < N && !differs; t += (long long) gridDim.x * blockDim.x) {
         Box b;
         b.lo[0] = b.lo[1] = b.lo[2] = 0;
         b.hi[0] = n0; b.hi[1] = n1; b.hi[2] = n2;
@@ -106,12 +109,20 @@ __global__ void class_check(const double* A, long long N, int n0, int n1, int n2
         box_index(t, b, i, j, k);
         auto pc = [](int x, int n) { return x == 0 ? 0 : (x == n - 1 ? 2 : 1); };
         const int cls = pc(i, n0) + 3 * (ndim > 1 ? pc(j, n1) : 0) + 9 * (ndim > 2 ? pc(k, n2) : 0);
-        for (int s = 0; s < NSLOT; ++s)
-            if (__double_as_longlong(A[s * N + t]) != __double_as_longlong(tab[cls * NSLOT + s])) { atomicExch(bad, 1); return; }
+        double v[NSLOT];
+#pragma unroll
+        for (int s = 0; s < NSLOT; ++s) v[s] = A[s * N + t];
+#pragma unroll
+        for (int s = 0; s < NSLOT; ++s) differs |= __double_as_longlong(v[s]) != __double_as_longlong(tab[cls * NSLOT + s]);
     }
+    // (a store of the same value by every warp that found one)
+    if (__any_sync(0xffffffffu, differs) && (threadIdx.x & 31) == 0) *(volatile int*) bad = 1;
 }
-// max |row sum| and max |diag| (bit patterns of non-negative doubles)
-__global__ void rowsum_stats(const double* A, long long N, int n0, int n1, int n2, int ndim, int p0, int p1, int p2, unsigned long long* out) {
+// max |row sum| and max |diag| (bit patterns of non-negative doubles); one pair of atomics per CTA (a pair per
+// thread held the same two addresses for 870 us at 192^3, now 118)
+__global__ void __launch_bounds__(256) rowsum_stats(const double* __restrict__ A, long long N, int n0, int n1, int n2, int ndim, int p0, int p1, int p2,
+                                                    unsigned long long* out) {
+    __shared__ unsigned long long sh[2][8];
     unsigned long long ms = 0, md = 0;
     for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < N; t += (long long) gridDim.x * blockDim.x) {
         Box b;
@@ -119,18 +130,36 @@ __global__ void rowsum_stats(const double* A, long long N, int n0, int n1, int n
         b.hi[0] = n0; b.hi[1] = n1; b.hi[2] = n2;
         int i, j, k;
         box_index(t, b, i, j, k);
-        double s = A[t];
         const int idx[3] = {i, j, k}, n[3] = {n0, n1, n2}, per[3] = {p0, p1, p2};
-        for (int d = 0; d < ndim; ++d) {
-            if (idx[d] > 0 || per[d]) s += A[(1 + 2 * d) * N + t];
-            if (idx[d] < n[d] - 1 || per[d]) s += A[(2 + 2 * d) * N + t];
+        double v[NSLOT];
+#pragma unroll
+        for (int s = 0; s < NSLOT; ++s) v[s] = s < 1 + 2 * ndim ? A[s * N + t] : 0.;
+        double s = v[0];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (d >= ndim) break;
+            if (idx[d] > 0 || per[d]) s += v[1 + 2 * d];
+            if (idx[d] < n[d] - 1 || per[d]) s += v[2 + 2 * d];
         }
-        const unsigned long long bs = (unsigned long long) __double_as_longlong(fabs(s)), bd = (unsigned long long) __double_as_longlong(fabs(A[t]));
+        const unsigned long long bs = (unsigned long long) __double_as_longlong(fabs(s)), bd = (unsigned long long) __double_as_longlong(fabs(v[0]));
         ms = bs > ms ? bs : ms;
         md = bd > md ? bd : md;
     }
-    atomicMax(&out[0], ms);
-    atomicMax(&out[1], md);
+    for (int w = 16; w > 0; w >>= 1) {
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, ms, w), c = __shfl_xor_sync(0xffffffffu, md, w);
+        ms = a > ms ? a : ms;
+        md = c > md ? c : md;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = ms;
+        sh[1][threadIdx.x >> 5] = md;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long m = 0;
+        for (int w = 0; w < 8; ++w) m = sh[threadIdx.x][w] > m ? sh[threadIdx.x][w] : m;
+        atomicMax(&out[threadIdx.x], m);
+    }
 }
 __global__ void sum_partials(const double* v, long long n, double* partial) {
     __shared__ double sh[256];
