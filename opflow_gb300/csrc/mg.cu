@@ -1164,10 +1164,27 @@ __global__ void __launch_bounds__(256) kr_zero_x(const LvlDev* __restrict__ Ls, 
     }
 }
 
-// p = z + beta p with z the V-cycle result (beta = 0 for the first direction)
+// the number of active problems, by one CTA
+__device__ __forceinline__ void count_active(const Scal* sc, int nprob, int* out) {
+    int c = 0;
+    for (int p = threadIdx.x; p < nprob; p += blockDim.x) c += sc[p].active;
+    for (int s = 16; s > 0; s >>= 1) c += __shfl_xor_sync(0xffffffffu, c, s);
+    __shared__ int sh[32];
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = 0;
+        for (int w = 0; w < (int) (blockDim.x >> 5); ++w) t += sh[w];
+        *out = t;
+    }
+}
+
+// p = z + beta p with z the V-cycle result (beta = 0 for the first direction); the count of active problems
+// for the loop's control alongside
 template <typename T>
 __global__ void __launch_bounds__(256) kr_pupdate(const LvlDev* __restrict__ Ls, const KrylovDev* __restrict__ K, const Chunk* __restrict__ ch, int nch,
-                                                  const Scal* sc, int first) {
+                                                  const Scal* sc, int first, int nprob, int* active_out) {
+    if (blockIdx.x == 0) count_active(sc, nprob, active_out);
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
         const Chunk C = ch[c];
         const LvlDev& L = Ls[C.lvl];
@@ -1229,20 +1246,6 @@ __global__ void kr_scalars(Scal* sc, const double* red, int nprob, int stage, do
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nprob) return;
     scalars_stage(sc[p], red[2 * p], red[2 * p + 1], stage, tol, max_iter, flexible);
-}
-
-__global__ void count_active(const Scal* sc, int nprob, int* out) {
-    int c = 0;
-    for (int p = threadIdx.x; p < nprob; p += blockDim.x) c += sc[p].active;
-    for (int s = 16; s > 0; s >>= 1) c += __shfl_xor_sync(0xffffffffu, c, s);
-    __shared__ int sh[32];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < (int) (blockDim.x >> 5); ++w) t += sh[w];
-        *out = t;
-    }
 }
 
 // ------------------------------------------------------------------------------------ launchers
@@ -1414,10 +1417,11 @@ int kr_launch_from_vcycle(cudaStream_t s, int sms, bool f32, const LvlDev* L, co
     OPG_LAUNCHED();
     return check_launch("kr_from_vcycle");
 }
-int kr_launch_pupdate(cudaStream_t s, int sms, bool f32, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch, const Scal* sc, int first) {
+int kr_launch_pupdate(cudaStream_t s, int sms, bool f32, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch, const Scal* sc, int first, int nprob,
+                      int* active_out) {
     if (nch <= 0) return OPFLOW_OK;
-    if (f32) kr_pupdate<float><<<grid_of(nch, sms), 256, 0, s>>>(L, K, ch, nch, sc, first);
-    else kr_pupdate<double><<<grid_of(nch, sms), 256, 0, s>>>(L, K, ch, nch, sc, first);
+    if (f32) kr_pupdate<float><<<grid_of(nch, sms), 256, 0, s>>>(L, K, ch, nch, sc, first, nprob, active_out);
+    else kr_pupdate<double><<<grid_of(nch, sms), 256, 0, s>>>(L, K, ch, nch, sc, first, nprob, active_out);
     OPG_LAUNCHED();
     return check_launch("kr_pupdate");
 }
@@ -1436,11 +1440,6 @@ int kr_launch_scalars(cudaStream_t s, Scal* sc, const double* red, int nprob, in
     kr_scalars<<<(nprob + 127) / 128, 128, 0, s>>>(sc, red, nprob, stage, tol, max_iter, flexible);
     OPG_LAUNCHED();
     return check_launch("kr_scalars");
-}
-int kr_launch_count(cudaStream_t s, const Scal* sc, int nprob, int* out) {
-    count_active<<<1, 256, 0, s>>>(sc, nprob, out);
-    OPG_LAUNCHED();
-    return check_launch("count_active");
 }
 
 }  // namespace opg

@@ -1,6 +1,9 @@
 // Launchers of the multigrid / Krylov kernels (mg.cu).
 #pragma once
 
+#include <array>
+#include <vector>
+
 #include <cuda.h>
 #include "mg.h"
 
@@ -50,15 +53,45 @@ int mg_launch_tile_up(cudaStream_t s, const LvlDev* L, const Chunk* strips, int 
 bool mg_vol_supported(int pre, int post);
 void mg_vol_tiles(int li, const LvlDev& D, int sweeps, int sms, int choice, std::vector<Chunk>& out);
 int mg_launch_vol(cudaStream_t s, const LvlDev* L, const Chunk* tiles, int n, const Scal* sc, int sweeps, bool down);
-// the V-cycle at and below each listed level of 2D problems whose levels there all take strips and whose
-// coarsest level has a dense inverse (pre = post = sweeps)
-constexpr int MG_BSTRIP_WARPS = 16, MG_BSTRIP_ROWS = 4;
-int mg_launch_bottom_strips(cudaStream_t s, const LvlDev* L, const int* top, int ntop, const Scal* sc, int sweeps);
 // the whole V-cycle below each listed level (a problem's first small level), one CTA per problem with
 // those levels' vectors in shared memory: at most MG_BOTTOM_LEVELS levels and MG_BOTTOM_CELLS cells
 // in all (`cells`: the largest such total of the listed problems)
 constexpr int MG_BOTTOM_LEVELS = 12;
 constexpr int MG_BOTTOM_CELLS = 8192;
+// the V-cycle at and below each listed level (mg_small.cu: float32 class-table levels with uniform off-diagonal
+// coefficients down to a dense coarsest solve), one CTA per problem; probs: the problems' levels laid out by
+// mg_small_problem, in the list's order; floats: the largest of their shared memory
+constexpr long long MG_SMALL_FLOATS = 51200;  // 200 KB of shared memory
+constexpr int MG_SMALL_SHARES = 5;            // warp shares (32 column pairs) that each of 32 warps holds of a level
+struct SmLevel {
+    int n[3], lo[3], per[3], glo[3], ghi[3];
+    int s1, s2;          // strides of rows and planes (cells, the ring of zeros included)
+    int x, b;            // places of cell (0, 0, 0)
+    int node;            // node-centred transfers to this level from the next finer one
+    int barrier;         // the level's named barrier
+    int lw;                        // a warp share: 2^lw column pairs of 32 / 2^lw rows
+    int half, pairs, shares;       // shares along a row, along the rows of a plane, in all
+    int lf, fgroups, frows;        // the same of single cells: 2^lf of 32 / 2^lf rows
+    unsigned mhalf, mrows, mfrows, mrow;  // quotients by half, pairs, frows and the rows of a plane
+    float c[6];          // off-diagonal coefficients
+    float c0[NCLASS], inv[NCLASS];
+};
+struct SmProblem {
+    const double* Ainv;
+    const float* b;      // the first level's vectors
+    float* x;
+    int problem, restricts;  // restricts: the finer level is not restricted into the first one yet
+    int ndim, levels, node, per;
+    int frames, lin;     // floats of the levels' x and b; place of the coarsest b in order (float64)
+    unsigned mn0;        // quotient by the first level's row
+    SmLevel lv[MG_BOTTOM_LEVELS];
+};
+struct SmSource {  // one level as mg_small_problem takes it
+    int ndim, n[3], lo[3], per[3], glo[3], ghi[3], node;
+    const std::vector<double>* tab;  // class table, NSLOT per class
+};
+bool mg_small_problem(const SmSource* L, int levels, const double* Ainv, SmProblem* P, long long* floats);
+int mg_launch_small(cudaStream_t s, const LvlDev* L, const int* top, const SmProblem* probs, int ntop, const Scal* sc, int pre, int post, long long floats);
 int mg_bottom_prepare();
 int mg_launch_bottom(cudaStream_t s, int sms, bool f32, const LvlDev* L, const int* top, int ntop, const Scal* sc, int pre, int post,
                      long long cells);
@@ -73,9 +106,9 @@ int kr_launch_update(cudaStream_t s, int sms, bool f32, const LvlDev* L, const K
                      const Finish& F = Finish{});
 int kr_launch_from_vcycle(cudaStream_t s, int sms, bool f32, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch, const Scal* sc,
                           double* partial, const Finish& F = Finish{});
-int kr_launch_pupdate(cudaStream_t s, int sms, bool f32, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch, const Scal* sc, int first);
+int kr_launch_pupdate(cudaStream_t s, int sms, bool f32, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch, const Scal* sc, int first,
+                      int nprob, int* active_out);
 int kr_launch_zero_x(cudaStream_t s, int sms, const LvlDev* L, const KrylovDev* K, const Chunk* ch, int nch);
 int kr_launch_reduce(cudaStream_t s, int sms, const double* partial, const int* first, const int* count, int nprob, double* out);
 int kr_launch_scalars(cudaStream_t s, Scal* sc, const double* red, int nprob, int stage, double tol, int max_iter, int flexible);
-int kr_launch_count(cudaStream_t s, const Scal* sc, int nprob, int* out);
 }  // namespace opg

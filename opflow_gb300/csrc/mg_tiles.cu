@@ -31,7 +31,7 @@
 // half of the issue slots used; 2.5 warp instructions per cell at 16 rows a strip), on small ones the
 // chain of half sweeps within a row (about 500 cycles).  Against the shared-memory tiles of 54 x 32 cells
 // it replaced: 2048^2 level 0 down 71 -> 24 us, up 114 -> 27 us; 18.5 M cells of 64 Helmholtz problems down
-// 460 -> 95 us, up 757 -> 131 us; levels of at most 32^2 cells (mg_bottom_strips) 51 -> 30 us.
+// 460 -> 95 us, up 757 -> 131 us.
 #include "mg_device.h"
 
 namespace opg {
@@ -55,7 +55,7 @@ __device__ __forceinline__ int wrap_pos(int g, int n) {
     return g < 0 ? g + n : g;
 }
 
-// Plain (coherent) loads: the bottom kernel reads what other warps of its CTA wrote before a barrier.
+// Plain (coherent) loads
 __device__ __forceinline__ float ldf(const float* p) { return __ldca(p); }
 
 // off-diagonal sum of the cell in column P (0: even, 1: odd) of a row: W and E from the row's other
@@ -453,52 +453,6 @@ __global__ void __launch_bounds__(32 * STRIP_WARPS) mg_strip(const LvlDev* __res
     if (mode == ROWS_INNER) strip_step<SW, DOWN, ROWS_INNER>(L, Lc, S, lane);
     else if (mode == ROWS_DIAG) strip_step<SW, DOWN, ROWS_DIAG>(L, Lc, S, lane);
     else strip_step<SW, DOWN, ROWS_GENERAL>(L, Lc, S, lane);
-}
-
-// The V-cycle at and below a 2D problem's first small level, one CTA per problem: every level's strips
-// (MG_BSTRIP_ROWS rows) spread over the CTA's warps, a barrier where the large levels have a launch
-// boundary, and the dense coarsest solve in between.  The levels' vectors stay in the L1 / L2 caches.
-// (Levels of which some row differs in more than its centre coefficient stay with mg_bottom.)
-template <int SW>
-__global__ void __launch_bounds__(32 * MG_BSTRIP_WARPS) mg_bottom_strips(const LvlDev* __restrict__ Ls, const int* __restrict__ top, const Scal* sc) {
-    const int s = top[blockIdx.x], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (sc && !sc[Ls[s].problem].active) return;
-    auto strips = [&](int l, bool down) {
-        const LvlDev& L = Ls[l];
-        const LvlDev& Lc = Ls[L.coarse];
-        const int node = Lc.node, hx = 2 * SW + node, w = 64 - 2 * hx;
-        const int first = node && ((L.lo[0] - hx) & 1) ? -1 : 0;
-        const int nx = (L.n[0] - first + w - 1) / w, ny = (L.n[1] + MG_BSTRIP_ROWS - 1) / MG_BSTRIP_ROWS;
-        for (int t = warp; t < nx * ny; t += MG_BSTRIP_WARPS) {
-            Chunk C{l, (t / nx) * MG_BSTRIP_ROWS, 0, first + (t % nx) * w, w};
-            C.nrows = MG_BSTRIP_ROWS;
-            const Strip S = strip_of(L, C, hx, 2 * SW + (down ? node : 0), lane);
-            if (down) strip_step<SW, true, ROWS_DIAG>(L, Lc, S, lane);
-            else strip_step<SW, false, ROWS_DIAG>(L, Lc, S, lane);
-        }
-        __syncthreads();
-    };
-    int l = s;
-    for (; !Ls[l].coarsest; l = Ls[l].coarse) strips(l, true);
-    coarse_rows<float>(Ls[l], threadIdx.x, blockDim.x);
-    __syncthreads();
-    while (l != s) {
-        l = Ls[l].fine;
-        strips(l, false);
-    }
-}
-
-int mg_launch_bottom_strips(cudaStream_t s, const LvlDev* L, const int* top, int ntop, const Scal* sc, int sweeps) {
-    if (ntop <= 0) return OPFLOW_OK;
-    switch (sweeps) {
-        case 1: mg_bottom_strips<1><<<ntop, 32 * MG_BSTRIP_WARPS, 0, s>>>(L, top, sc); break;
-        case 2: mg_bottom_strips<2><<<ntop, 32 * MG_BSTRIP_WARPS, 0, s>>>(L, top, sc); break;
-        case 3: mg_bottom_strips<3><<<ntop, 32 * MG_BSTRIP_WARPS, 0, s>>>(L, top, sc); break;
-        case 4: mg_bottom_strips<4><<<ntop, 32 * MG_BSTRIP_WARPS, 0, s>>>(L, top, sc); break;
-        default: return fail(OPFLOW_E_INVALID, "mg_bottom_strips: %d sweeps", sweeps);
-    }
-    OPG_LAUNCHED();
-    return check_launch("mg_bottom_strips");
 }
 
 bool mg_tiles_supported(int sweeps) { return sweeps >= 1 && sweeps <= MG_STRIP_SWEEPS; }

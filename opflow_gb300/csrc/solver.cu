@@ -750,7 +750,9 @@ int mg_finalize(MGSystem* S) {
     S->coarse_sm_ch.clear();
     S->bottom_host.clear();
     S->bottom_cells_host.clear();
-    S->bstrip_host.clear();
+    S->small_host.clear();
+    S->small_probs.clear();
+    S->small_floats = 0;
     OPG_TRY(mg_bottom_prepare());
     const char* te = getenv("OPFLOW_MG_TILES");
     // strips for the float32 V-cycle only: the float64 one is bound by float64 issue, where the halo's
@@ -782,7 +784,7 @@ int mg_finalize(MGSystem* S) {
                 out.push_back(c);
             }
     };
-    if (const char* e = getenv("OPFLOW_MG_BOTTOM")) S->bottom_max = S->bstrip_max = atoll(e);
+    if (const char* e = getenv("OPFLOW_MG_BOTTOM")) S->bottom_max = S->small_max2 = S->small_max3 = atoll(e);
     // level-0 chunks of the Krylov kernels: whole rows of one plane, about KCH cells each (rows longer
     // than KCH are split), so the per-chunk reduction and its barriers are amortised over many cells.
     // KCH is 8192 for problems of at least 8192 cells per two SMs and halves (down to 1024) for smaller
@@ -844,15 +846,42 @@ int mg_finalize(MGSystem* S) {
             }
             return true;
         };
-        // first level small enough for a one-CTA bottom kernel (levels.size(): none): the strips' where every
-        // level from there on takes them down to a dense coarsest solve, else the per-cell one
+        // first level small enough for a one-CTA kernel (levels.size(): none): mg_small where every level from
+        // there on takes it down to a dense coarsest solve, else the per-cell one
         size_t sp = P.levels.size();
-        for (size_t l = 0; l < P.levels.size(); ++l)
-            if (P.levels[l].N <= S->bstrip_max) { sp = l; break; }
-        bool bstrip = S->pre == S->post && P.levels.back().Ainv64 && sp + 1 < P.levels.size() && (sp == 0 || stripable(sp - 1));
-        for (size_t l = sp; bstrip && l + 1 < P.levels.size(); ++l) bstrip = stripable(l) && P.levels[l].uoff;
+        SmProblem sprob;
+        long long sfloats = 0;
+        const bool smallable = f32 && tiles_on && S->pre >= 1 && P.levels.back().Ainv64 && P.levels.back().ndim >= 2;
+        for (size_t l = P.levels.size() - 1; smallable && l-- > 0;) {
+            const LevelHost &F = P.levels[l], &Cn = P.levels[l + 1];
+            bool ok = F.table && F.uoff && F.N <= (F.ndim == 2 ? S->small_max2 : S->small_max3);
+            for (int d = 0; d < F.ndim; ++d) ok = ok && !(F.per[d] && (F.n[d] & 1)) && (Cn.node || Cn.n[d] == (F.n[d] + 1) / 2);
+            std::vector<SmSource> src;
+            for (size_t q = l; q < P.levels.size(); ++q) {
+                const LevelHost& H = P.levels[q];
+                SmSource X{};
+                X.ndim = H.ndim;
+                for (int d = 0; d < 3; ++d) {
+                    X.n[d] = H.n[d];
+                    X.lo[d] = d < H.ndim ? H.lo[d] : 0;
+                    X.per[d] = H.per[d];
+                    X.glo[d] = H.gh_lo[d];
+                    X.ghi[d] = H.gh_hi[d];
+                }
+                X.node = H.node;
+                X.tab = &H.tab;
+                src.push_back(X);
+            }
+            SmProblem at;
+            long long fl = 0;
+            if (!ok || !mg_small_problem(src.data(), (int) src.size(), P.levels.back().Ainv64, &at, &fl)) break;
+            sp = l;
+            sprob = at;
+            sfloats = fl;
+        }
+        const bool small = sp < P.levels.size();
         long long bcells = 0;
-        if (!bstrip) {
+        if (!small) {
             sp = P.levels.size();
             for (size_t l = 0; l < P.levels.size(); ++l)
                 if (P.levels[l].N <= S->bottom_max) { sp = l; break; }
@@ -912,8 +941,14 @@ int mg_finalize(MGSystem* S) {
             }
             lv.push_back(D);
             const int li = base + (int) l;
-            if (l == sp && bstrip) {
-                S->bstrip_host.push_back(li);
+            if (l == sp && small) {
+                S->small_host.push_back(li);
+                sprob.b = D.b32;
+                sprob.x = D.x32;
+                sprob.problem = (int) p;
+                sprob.restricts = l > 0 && !tileable(l - 1);
+                S->small_probs.push_back(sprob);
+                S->small_floats = std::max(S->small_floats, sfloats);
             } else if (l == sp) {
                 S->bottom_host.push_back(li);
                 S->bottom_cells_host.push_back(bcells);
@@ -1024,11 +1059,13 @@ int mg_finalize(MGSystem* S) {
     S->bottom_cells = 0;
     for (long long c : S->bottom_cells_host) S->bottom_cells = std::max(S->bottom_cells, c);
     S->dbottom = (int*) S->arena.alloc(std::max<size_t>(1, S->bottom_host.size()) * sizeof(int));
-    S->nbstrip = (int) S->bstrip_host.size();
-    S->dbstrip = (int*) S->arena.alloc(std::max<size_t>(1, S->bstrip_host.size()) * sizeof(int));
-    if (!S->dbottom || !S->dbstrip) return fail(OPFLOW_E_NOMEM, "solver tables");
+    S->nsmall = (int) S->small_host.size();
+    S->dsmall = (int*) S->arena.alloc(std::max<size_t>(1, S->small_host.size()) * sizeof(int));
+    S->dsmall_probs = (SmProblem*) S->arena.alloc(std::max<size_t>(1, S->small_probs.size()) * sizeof(SmProblem));
+    if (!S->dbottom || !S->dsmall || !S->dsmall_probs) return fail(OPFLOW_E_NOMEM, "solver tables");
     if (S->nbottom) cudaMemcpyAsync(S->dbottom, S->bottom_host.data(), S->bottom_host.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
-    if (S->nbstrip) cudaMemcpyAsync(S->dbstrip, S->bstrip_host.data(), S->bstrip_host.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+    if (S->nsmall) cudaMemcpyAsync(S->dsmall_probs, S->small_probs.data(), S->small_probs.size() * sizeof(SmProblem), cudaMemcpyHostToDevice, ctx->stream);
+    if (S->nsmall) cudaMemcpyAsync(S->dsmall, S->small_host.data(), S->small_host.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
     if (!S->dL || !S->dK || !S->dS || !S->dk0 || !S->partial || !S->red || !S->dcoarse) return fail(OPFLOW_E_NOMEM, "solver tables");
     cudaMemcpyAsync(S->dL, lv.data(), lv.size() * sizeof(LvlDev), cudaMemcpyHostToDevice, ctx->stream);
     cudaMemcpyAsync(S->dK, kd.data(), kd.size() * sizeof(KrylovDev), cudaMemcpyHostToDevice, ctx->stream);
@@ -1118,7 +1155,7 @@ static int vcycle(MGSystem* S) {
         OPG_TRY(mg_launch_residual(s, sms, f32, S->dL, C.ptr, C.n, sc));
         OPG_TRY(mg_launch_residual_z(s, sms, f32, S->dL, Z.ptr, Z.n, sc, S->zb[l]));
     }
-    OPG_TRY(mg_launch_bottom_strips(s, S->dL, S->dbstrip, S->nbstrip, sc, S->pre));
+    OPG_TRY(mg_launch_small(s, S->dL, S->dsmall, S->dsmall_probs, S->nsmall, sc, S->pre, S->post, S->small_floats));
     OPG_TRY(mg_launch_bottom(s, sms, f32, S->dL, S->dbottom, S->nbottom, sc, S->pre, S->post, S->bottom_cells));
     OPG_TRY(mg_launch_coarse(s, sms, f32, S->dL, S->dcoarse, S->ncoarse, sc));
     for (int it = 0; it < S->pre + S->post; ++it) {
@@ -1169,8 +1206,7 @@ static int iteration(MGSystem* S, bool readback) {
     OPG_TRY(kr_launch_update(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, S->partial, finish(S, 2)));
     OPG_TRY(vcycle(S));
     OPG_TRY(kr_launch_from_vcycle(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, S->partial, finish(S, 3)));
-    OPG_TRY(kr_launch_pupdate(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, 0));
-    OPG_TRY(kr_launch_count(s, S->dS, np, S->d_active));
+    OPG_TRY(kr_launch_pupdate(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, 0, np, S->d_active));
     if (readback) OPG_CUDA(cudaMemcpyAsync(S->h_active, S->d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
     return OPFLOW_OK;
 }
@@ -1184,8 +1220,7 @@ static int first_direction(MGSystem* S) {
     OPG_TRY(kr_launch_apply(s, sms, S->dL, S->dK, S->dk0, S->nk0, nullptr, S->partial, 0, finish(S, 0), 1, f32));
     OPG_TRY(vcycle(S));
     OPG_TRY(kr_launch_from_vcycle(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, S->partial, finish(S, 4)));
-    OPG_TRY(kr_launch_pupdate(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, 1));
-    return kr_launch_count(s, S->dS, np, S->d_active);
+    return kr_launch_pupdate(s, sms, f32, S->dL, S->dK, S->dk0, S->nk0, S->dS, 1, np, S->d_active);
 }
 
 // Loop control of the whole-solve graph.  Before the loop (reset) the counter starts at 0; after each
@@ -1377,9 +1412,10 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     std::vector<LvlDev> lv;
     std::vector<KrylovDev> kd;
     std::vector<Chunk> k0;
-    std::vector<int> first, count, coarse_list, bottom_list, bstrip_list;
+    std::vector<int> first, count, coarse_list, bottom_list, small_list;
     std::vector<long long> bottom_cells;
-    C->bottom_cells = 0;
+    C->bottom_cells = C->small_floats = 0;
+    C->small_probs.clear();
     C->nlevels = 0;
     for (auto* P : parts) C->nlevels = std::max(C->nlevels, P->nlevels);
     C->smooth_ch.assign(C->nlevels, {});
@@ -1412,7 +1448,12 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
         }
         for (int c : P->coarse_host) coarse_list.push_back(base + c);
         for (int b : P->bottom_host) bottom_list.push_back(base + b);
-        for (int b : P->bstrip_host) bstrip_list.push_back(base + b);
+        for (int b : P->small_host) small_list.push_back(base + b);
+        for (SmProblem sp : P->small_probs) {
+            sp.problem = (int) q;
+            C->small_probs.push_back(sp);
+        }
+        C->small_floats = std::max(C->small_floats, P->small_floats);
         for (long long c : P->bottom_cells_host) {
             bottom_cells.push_back(c);
             C->bottom_cells = std::max(C->bottom_cells, c);
@@ -1460,14 +1501,16 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     C->bottom_cells_host = bottom_cells;
     C->nbottom = (int) bottom_list.size();
     C->dbottom = (int*) C->arena.alloc(std::max<size_t>(1, bottom_list.size()) * sizeof(int));
-    C->bstrip_host = bstrip_list;
-    C->nbstrip = (int) bstrip_list.size();
-    C->dbstrip = (int*) C->arena.alloc(std::max<size_t>(1, bstrip_list.size()) * sizeof(int));
+    C->small_host = small_list;
+    C->nsmall = (int) small_list.size();
+    C->dsmall = (int*) C->arena.alloc(std::max<size_t>(1, small_list.size()) * sizeof(int));
+    C->dsmall_probs = (SmProblem*) C->arena.alloc(std::max<size_t>(1, small_list.size()) * sizeof(SmProblem));
     C->d_active = (int*) C->arena.alloc(2 * sizeof(int));
     C->d_done = (int*) C->arena.alloc(np * sizeof(int));
     if (!C->d_done) return fail(OPFLOW_E_NOMEM, "batch tables");
     cudaMemsetAsync(C->d_done, 0, np * sizeof(int), ctx->stream);
-    if (!C->dL || !C->dK || !C->dS || !C->dk0 || !C->dfirst || !C->dcount || !C->partial || !C->red || !C->dcoarse || !C->d_active || !C->dbottom || !C->dbstrip)
+    if (!C->dL || !C->dK || !C->dS || !C->dk0 || !C->dfirst || !C->dcount || !C->partial || !C->red || !C->dcoarse || !C->d_active || !C->dbottom || !C->dsmall ||
+        !C->dsmall_probs)
         return fail(OPFLOW_E_NOMEM, "batch tables");
     cudaStream_t s = ctx->stream;
     if (!lv.empty()) cudaMemcpyAsync(C->dL, lv.data(), lv.size() * sizeof(LvlDev), cudaMemcpyHostToDevice, s);
@@ -1478,7 +1521,8 @@ int mg_compose(MGSystem* C, const std::vector<MGSystem*>& parts, const std::vect
     if (!count.empty()) cudaMemcpyAsync(C->dcount, count.data(), count.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (!coarse_list.empty()) cudaMemcpyAsync(C->dcoarse, coarse_list.data(), coarse_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (!bottom_list.empty()) cudaMemcpyAsync(C->dbottom, bottom_list.data(), bottom_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
-    if (!bstrip_list.empty()) cudaMemcpyAsync(C->dbstrip, bstrip_list.data(), bstrip_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
+    if (!small_list.empty()) cudaMemcpyAsync(C->dsmall_probs, C->small_probs.data(), C->small_probs.size() * sizeof(SmProblem), cudaMemcpyHostToDevice, s);
+    if (!small_list.empty()) cudaMemcpyAsync(C->dsmall, small_list.data(), small_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     auto upload = [&](std::vector<Chunk>& h, ChunkList& d) {
         d.n = (int) h.size();
         d.ptr = (Chunk*) C->arena.alloc(std::max<size_t>(1, h.size()) * sizeof(Chunk));

@@ -105,13 +105,17 @@ struct MGSystem {
     std::vector<int> coarse_host, bottom_host;
     int* dbottom = nullptr;
     int nbottom = 0;
-    // 2D problems whose small levels all take strips: their first level of at most bstrip_max cells instead
-    // (mg_bottom_strips).  Of 1024, 4096, 16384: 2048^2 solve 3.88, 3.94, 4.40 ms (64^2 is quicker as a launch
-    // of its own), a served mix of 24 requests with levels of 45^2 to 55^2 261, 257, 278 ms.
-    long long bstrip_max = 3072;
-    std::vector<int> bstrip_host;
-    int* dbstrip = nullptr;
-    int nbstrip = 0;
+    // Problems whose small levels mg_small takes: their first level of at most small_max2 (2D) or small_max3 (3D)
+    // cells instead.  Measured, 2D with 1100, 3072, 6400, 9216 cells: 2048^2 solve (a level of 64^2) 3.09, 3.09,
+    // 3.01, 3.01 ms, a served mix of 24 requests 190, 180, 186, 187 ms (levels of 70^2 to 90^2 are quicker as
+    // strips); 3D with 600, 4096, 8000: 256^3 (16^3) 8.88, 8.77, 8.77 ms.
+    long long small_max2 = 4352, small_max3 = 4096;
+    std::vector<int> small_host;
+    std::vector<SmProblem> small_probs;  // laid out for the kernel, in small_host's order
+    int* dsmall = nullptr;
+    SmProblem* dsmall_probs = nullptr;
+    int nsmall = 0;
+    long long small_floats = 0;  // largest shared memory of those problems, in floats
     long long bottom_cells = 0;  // largest cell total of a problem's bottom levels (shared memory of mg_bottom)
     std::vector<long long> bottom_cells_host;  // per entry of bottom_host
     std::vector<KrylovDev> kd_host;
