@@ -41,8 +41,8 @@ __device__ __forceinline__ void chunk_cells(const Chunk& C, int color, F&& f) {
     }
 }
 
-// A chunk of a level with coefficient arrays: the cells of one colour updated (color 0, 1), or the residual of
-// all (color -1).  Threads take cells one after another over the whole chunk, so that short rows leave none
+// A chunk of a level with coefficient arrays: the cells of one colour updated (color 0, 1), those of colour 0
+// from x = 0 (color 2: x = b / c0, two arrays instead of nine: 49 us at 192^3), or the residual of all (color -1).  Threads take cells one after another over the whole chunk, so that short rows leave none
 // idle.  It is bound by the bytes (a half sweep reads every sector of the 2 ND + 1 arrays) and, in float64, the
 // pipe (13 operations per updated cell, the quotient's six among them).  192^3, 3D: half sweep 212 -> 96 us, residual
 // 337 -> 116 us against one load in flight per thread and the compiler's division.
@@ -59,7 +59,13 @@ static __device__ __noinline__ void array_chunk(const LvlDev& L, const Chunk C, 
     for (int it = threadIdx.x; it < half * C.nrows; it += blockDim.x) {
         const int r = it / half, j = C.j + r;
         const int t = 2 * (it - r * half) + ((C.i0 + j + C.k + color) & 1);
-        if (t < C.cnt) array_cell<T, ND, true>(L, C.i0 + t, j, C.k);
+        if (t >= C.cnt) continue;
+        if (color == 2) {
+            const long long cell = cell_of(L, C.i0 + t, j, C.k);
+            Sel<T>::x(L)[cell] = quotient(Sel<T>::b(L)[cell], Sel<T>::A(L)[cell]);
+        } else {
+            array_cell<T, ND, true>(L, C.i0 + t, j, C.k);
+        }
     }
 }
 template <typename T>
@@ -81,7 +87,8 @@ __global__ void __launch_bounds__(256, 4) mg_residual(const LvlDev* __restrict__
 }
 
 // Red-black Gauss-Seidel half sweep (cells with (i+j+k)%2 == color), or for Jacobi levels:
-// color 0 computes r = b - A x, color 1 applies x += omega r / diag.
+// color 0 computes r = b - A x, color 1 applies x += omega r / diag.  color 2: colour 0 where x is 0 (a
+// V-cycle's first half sweep on a level).
 template <typename T>
 __global__ void __launch_bounds__(256, 4) mg_smooth(const LvlDev* __restrict__ Ls, const Chunk* __restrict__ ch, int nch, int color, const Scal* sc) {
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
@@ -89,8 +96,8 @@ __global__ void __launch_bounds__(256, 4) mg_smooth(const LvlDev* __restrict__ L
         if (!active(Ls, C, sc)) continue;
         const LvlDev& L = Ls[C.lvl];
         if (L.rbgs && !L.table) array_level<T>(L, C, color);
-        else if (L.rbgs) chunk_cells(C, color, [&](int i, int j) { cell_gs<T>(L, i, j, C.k); });
-        else chunk_cells(C, -1, [&](int i, int j) { cell_jacobi<T>(L, i, j, C.k, color); });
+        else if (L.rbgs) chunk_cells(C, color & 1, [&](int i, int j) { cell_gs<T>(L, i, j, C.k); });
+        else chunk_cells(C, -1, [&](int i, int j) { cell_jacobi<T>(L, i, j, C.k, color & 1); });
     }
 }
 

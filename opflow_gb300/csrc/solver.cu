@@ -1147,7 +1147,7 @@ static int vcycle(MGSystem* S) {
         const ChunkList& C = S->d_smooth[l];
         const ChunkList& Z = S->d_zsm[l];
         for (int it = 0; it < S->pre; ++it) {
-            OPG_TRY(mg_launch_smooth(s, sms, f32, S->dL, C.ptr, C.n, 0, sc));
+            OPG_TRY(mg_launch_smooth(s, sms, f32, S->dL, C.ptr, C.n, it == 0 ? 2 : 0, sc));
             OPG_TRY(smooth_z_level(S, l, 0));
             OPG_TRY(mg_launch_smooth(s, sms, f32, S->dL, C.ptr, C.n, 1, sc));
             OPG_TRY(smooth_z_level(S, l, 1));
