@@ -718,22 +718,36 @@ __global__ void __launch_bounds__(256) fast_stencil_kernel(FieldView in, FieldVi
     }
 }
 
-// max |u| over a box, as the bit pattern of a non-negative double
-__global__ void maxabs_kernel(FieldView in, Box box, unsigned long long* slot) {
-    const long long nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1], nz = box.hi[2] - box.lo[2];
-    const long long total = nx * ny * nz;
+// max |u| over n values, as the bit pattern of a non-negative double.  Bound by the bytes: eight loads in flight
+// per thread and one atomic per CTA (512^3: 546 -> 171 us against an index division per load and an atomic per
+// warp).
+__global__ void __launch_bounds__(256) maxabs_kernel(const double* __restrict__ v, long long n, unsigned long long* slot) {
+    __shared__ unsigned long long sh[8];
     unsigned long long m = 0;
-    for (long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x; t < total; t += (long long) gridDim.x * blockDim.x) {
-        int i, j, k;
-        box_index(t, box, i, j, k);
-        const unsigned long long b = (unsigned long long) __double_as_longlong(ld(in, i, j, k)) & 0x7FFFFFFFFFFFFFFFull;
+    const long long step = (long long) gridDim.x * blockDim.x;
+    long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+    auto take = [&](double x) {
+        const unsigned long long b = (unsigned long long) __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
         m = b > m ? b : m;
+    };
+    for (; t + 7 * step < n; t += 8 * step) {
+        double x[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = v[t + q * step];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) take(x[q]);
     }
+    for (; t < n; t += step) take(v[t]);
     for (int s = 16; s > 0; s >>= 1) {
-        const unsigned long long o2 = __shfl_xor_sync(0xffffffffu, m, s);
-        m = o2 > m ? o2 : m;
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, s);
+        m = o > m ? o : m;
     }
-    if ((threadIdx.x & 31) == 0) atomicMax(slot, m);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
+        atomicMax(slot, m);
+    }
 }
 
 // ======================================================================================== small kernels
@@ -1313,9 +1327,9 @@ int opflow_assign_repeat(opflow_ctx ctx, opflow_field dst, int arith, const opfl
         cudaMemsetAsync(maxslots, 0, 3 * sizeof(unsigned long long), ctx->stream);
         // the source's readable values bound the fixed-point scale of the first step
         const opflow_field src = leaves[plan.src_slot];
-        Box all;
-        for (int d = 0; d < 3; ++d) { all.lo[d] = src->info.data_offset[d]; all.hi[d] = all.lo[d] + src->info.data_dims[d]; }
-        maxabs_kernel<<<grid_for(ctx, all.count(), 256), 256, 0, ctx->stream>>>(src->view(), all, maxslots);
+        const FieldView sv = src->view();  // (rows and planes without gaps)
+        const long long n = sv.sz * sv.dims[2];
+        maxabs_kernel<<<grid_for(ctx, n, 256 * 8), 256, 0, ctx->stream>>>(sv.data, n, maxslots);
         OPG_LAUNCHED();
         rc = check_launch("maxabs_kernel");
         if (rc) { free_plan(ctx, &plan); return rc; }
