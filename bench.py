@@ -144,13 +144,13 @@ def ftcs_kernel_label(D, mode, steps):
     if D == 2:
         if resident:
             return "axis2d_fxres_kernel<0> (resident fixed-point run; its first step converts float64 in, its last float64 out)"
-        return "axis2d_kernel<FAST>" if mode == "fast" else "axis2d_kernel<EXACT>"
+        return "axis2d_kernel<FAST>" if mode == "fast" else "axis_exact_kernel"
     if resident and os.environ.get("OPFLOW_FXRES_TMA", "1") != "0":
         return ("axis3d_fxtma_kernel (resident fixed-point run, planes staged in shared memory by TMA; its first and last steps "
                 "run axis3d_fxres_kernel<1|2, 6>: float64 in, float64 out)")
     if resident:
         return "axis3d_fxres_kernel<0, 6> (resident fixed-point run; its first step converts float64 in, its last float64 out)"
-    return "axis3d_rb_kernel<FAST>" if mode == "fast" else "axis3d_kernel<EXACT>"
+    return "axis3d_rb_kernel<FAST>" if mode == "fast" else "axis_exact_kernel"
 
 
 def replica_max(x, world, dist, device):

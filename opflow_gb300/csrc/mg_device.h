@@ -1,5 +1,5 @@
-// Device-side pieces of the multigrid V-cycle shared by the chunked kernels (mg.cu), the bottom kernel
-// (mg.cu) and the tile kernels (mg_tiles.cu): operator access and the per-cell bodies of smoothing,
+// Device-side pieces of the multigrid V-cycle shared by the chunked kernels and the bottom kernel (mg.cu) and
+// the fused steps (mg_tiles.cu, mg_vol.cu, mg_small.cu): operator access and the per-cell bodies of smoothing,
 // residual, restriction and prolongation.
 #pragma once
 #include "f64div.h"

@@ -698,7 +698,7 @@ static int tune_levels(MGSystem* S) {
             }
         }
         if (!S->tile_alt[l].empty()) {
-            // candidate 0: the list built (the shape the SM-fill rule picked), 1: the other shape
+            // candidate 0: the list built (the rows the fill rule picked), 1: the other rows
             ChunkList alt{};
             const int pick = choose(level_key("mg_tile", S, l), {0, 1}, [&](int cand) {
                 if (cand == 1 && !alt.ptr) {
