@@ -27,6 +27,17 @@ def _mesh(dims, stretched):
     return cm.mesh_points([cm.stretched_points(n) for n in dims]) if stretched else cm.mesh_uniform(list(dims))
 
 
+def _terms(u, K, n):
+    return [(u + 0.01 * (q + 1)) * (K - 0.02 * (q + 1)) / (3.0 + q) for q in range(n)]
+
+
+def _sum(ts):
+    s = ts[0]
+    for t in ts[1:]:
+        s = s + t
+    return s
+
+
 EXPRS = {
     "transport": lambda u, K, d: u + 1e-5 * sum((api.d1(api.d1IntpCenterToCorner(K, q) * api.d1(u, q), q) for q in range(1, d)),
                                                 api.d1(api.d1IntpCenterToCorner(K, 0) * api.d1(u, 0), 0)) - 0.3 * api.d1_biased_upwind(u, 0),
@@ -62,6 +73,32 @@ def test_expressions_match_the_oracle(ctx, dims, stretched, name):
             orc.assign(hu, nodes, [hu, hk], op)
             got, want = u.download(), hu.data
             assert np.array_equal(got, want, equal_nan=True), (values.__name__, op, np.nanmax(np.abs(got - want)))
+
+
+LONG = {
+    # more than a small launch's instructions, more than any launch's, and more values at once than places
+    "long": lambda u, K: _sum(_terms(u, K, 50)),
+    "too_long": lambda u, K: _sum(_terms(u, K, 190)),
+    "too_many": lambda u, K: _sum(_terms(u, K, 60)) * _sum([t * K for t in _terms(u, K, 60)]),
+}
+
+
+@pytest.mark.parametrize("dims", [(70, 37), (45, 33, 40)])
+@pytest.mark.parametrize("name", sorted(LONG))
+def test_long_expressions_match_numpy(ctx, dims, name):
+    # (element by element: numpy's IEEE operations in the same order)
+    mesh = _mesh(dims, False)
+    fd = cm.field_desc(len(dims), capi.CENTER, [(capi.BC_NEUM, capi.BC_NEUM)] * len(dims), ext=1)
+    u, K = api.CartesianField(mesh, fd, ctx), api.CartesianField(mesh, fd, ctx)
+    sl = u.index_slices(u.assignableRange)
+    vals = []
+    for f in (u, K):
+        a = f.download()
+        a[sl] = _uniform(np.random.default_rng(len(vals)), a[sl].shape)
+        f.upload(a)
+        vals.append(a[sl].copy())
+    u.assign(LONG[name](u, K))
+    assert np.array_equal(u.download()[sl], LONG[name](*vals))
 
 
 @pytest.mark.parametrize("n,stretched", [([80, 70], False), ([80, 70], True), ([260, 150], True), ([20, 21, 22], False), ([36, 33, 40], True)])
