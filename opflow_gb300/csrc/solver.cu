@@ -813,18 +813,19 @@ int mg_finalize(MGSystem* S) {
     // STRIP_FILL strips per SM.  Tall strips recompute fewer halo rows, short ones keep more warps on a
     // small level, where a step takes as long as one strip's march.  2048^2 solve / batch of 64 Helmholtz
     // problems (18.5 M cells) with 4, 8, 16, 32 strips per SM: 4.43, 4.39, 4.33, 4.33 / 11.6, 11.3, 11.1,
-    // 10.9 ms.
+    // 10.9 ms.  At least 4 rows (a march of 12): with 8, 4, 2 the 2048^2 solve takes 3.04, 2.95, 2.93 ms, a served
+    // mix of 24 requests 179.5, 175.0, 177.0 ms, the batch 9.21, 9.19, 9.23 ms.
     auto strip_rows = [&](size_t l) {
-        const int STRIP_FILL = 32;
+        const int STRIP_FILL = 32, LEAST = 4;
         const int w = 64 - 4 * std::max(S->pre, S->post);
-        for (int rows = 64; rows > 8; rows /= 2) {
+        for (int rows = 64; rows > LEAST; rows /= 2) {
             long long n = 0;
             for (const ProblemHost& P : S->probs)
                 if (l < P.levels.size() && P.levels[l].ndim == 2)
                     n += (long long) ((P.levels[l].n[0] + w - 1) / w) * ((P.levels[l].n[1] + rows - 1) / rows);
             if (n >= (long long) STRIP_FILL * ctx->num_sms) return rows;
         }
-        return 8;
+        return LEAST;
     };
     for (size_t p = 0; p < S->probs.size(); ++p) {
         ProblemHost& P = S->probs[p];
