@@ -77,3 +77,16 @@ def test_array_levels_scaled_to_the_ends_of_the_range(ctx, n, k):
     got = _solve(ctx, n, "dirc", True, "fp64", guess=False, A=2.0 ** k)
     assert got[0].niter == want[0].niter
     assert np.array_equal(got[2], want[2] * 2.0 ** -k)
+
+
+@pytest.mark.parametrize("n,bc", [
+    ([9, 1], "per"), ([1, 9], "per"), ([300, 1], "per"), ([1, 1], "per"),
+    ([9, 1, 8], "per"), ([1, 8, 9], "per"), ([40, 9, 1], "per"), ([70, 1, 50], "per"), ([7, 1, 1], "per"),
+    ([9, 1], "neum"), ([1, 9], "neum"), ([9, 1, 8], "neum"), ([40, 9, 1], "dirc"),
+])
+@pytest.mark.parametrize("array", [False, True])
+def test_directions_of_one_cell(ctx, n, bc, array):
+    # a periodic direction of one cell: the cell is its own neighbour on both sides
+    for prec in ("mixed", "fp64"):
+        st, res, _ = _solve(ctx, n, bc, array, prec)
+        assert st.converged and res <= 1.001 * TOL, (prec, st, res)
