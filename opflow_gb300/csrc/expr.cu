@@ -1391,8 +1391,9 @@ int opflow_assign_batch(opflow_ctx ctx, int n, const opflow_field* dsts, const i
             // the items' tiles march as far as leaves the whole batch its share of tiles per SM
             const Box& b = plans[i].box;
             const long long total = b.count();
-            const int m = D - 1, march = exact_march(b, D, ctx->num_sms, (double) total / (double) std::max(1LL, xcells));
-            for (int a = b.lo[m]; total > 0 && a < b.hi[m]; a += march)
+            if (total == 0) continue;
+            const int m = D - 1, march = exact_march(b, D, ctx->num_sms, (double) total / (double) xcells);
+            for (int a = b.lo[m]; a < b.hi[m]; a += march)
                 for (int y0 = b.lo[1]; y0 < (D == 3 ? b.hi[1] : b.lo[1] + 1); y0 += EX_ROWS)
                     for (int x0 = b.lo[0]; x0 < b.hi[0]; x0 += EX_COLS) xtiles.push_back(ExactTile{i, x0, y0, a, std::min(a + march, b.hi[m])});
         }

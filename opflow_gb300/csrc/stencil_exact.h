@@ -182,7 +182,7 @@ __host__ __device__ __forceinline__ void exact_dispatch(int mode, F&& f) {
 inline int exact_march(const Box& box, int ndim, int sms, double share) {
     const long long want = (long long) (share * sms * (ndim == 3 ? EX_FILL3 : EX_FILL));
     const long long nx = box.hi[0] - box.lo[0], ny = box.hi[1] - box.lo[1], nz = box.hi[2] - box.lo[2];
-    const long long across = (nx + EX_COLS - 1) / EX_COLS * (ndim == 3 ? (ny + EX_ROWS - 1) / EX_ROWS : 1);
+    const long long across = std::max(1LL, (nx + EX_COLS - 1) / EX_COLS * (ndim == 3 ? (ny + EX_ROWS - 1) / EX_ROWS : 1));  // (an empty box has none)
     const long long len = ndim == 3 ? nz : ny;
     const long long runs = std::max(1LL, (want + across - 1) / across);
     return (int) std::max(4LL, std::min(32LL, (len + runs - 1) / runs));

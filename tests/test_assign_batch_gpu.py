@@ -55,6 +55,17 @@ def test_batch_equals_each_assignment_alone(ctx, steps):
         assert np.array_equal(dst.download(), want[k]), k
 
 
+def test_batch_with_grids_without_an_inner_node(ctx):
+    # two Dirichlet nodes along a direction: nothing to assign, beside grids that have something
+    dims = [(2, 8), (33, 20), (8, 2, 8), (8, 2), (9, 8, 7), (8, 8, 2)]
+    sets = [[_field(ctx, d, capi.CORNER, capi.BC_DIRC, k) for k, d in enumerate(dims)] for _ in range(2)]
+    for u in sets[0]:
+        u.assign(cm.ftcs_expr(u, 1e-3, len(u.download().shape)), mode="exact", steps=2)
+    api.assign_batch([(u, cm.ftcs_expr(u, 1e-3, len(u.download().shape))) for u in sets[1]], steps=2)
+    for a, b in zip(*sets):
+        assert np.array_equal(a.download(), b.download())
+
+
 def test_batch_misuse_is_refused(ctx):
     u = _field(ctx, (33, 33), capi.CORNER, capi.BC_DIRC, 1)
     v = _field(ctx, (33, 33), capi.CORNER, capi.BC_DIRC, 2)

@@ -1,0 +1,68 @@
+"""The library's host side over a CUDA runtime without a device (tests/fake_cuda): calls that have to
+survive, and what they allocate, upload and wait for.  Each runs in a process of its own."""
+import glob
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HEAD = """
+import ctypes as C, sys
+sys.path[:0] = %r
+from opflow_gb300 import _capi as capi
+capi.LIB_PATH = sys.argv[1]
+from opflow_gb300 import api
+import common as cm
+count = lambda name: C.c_int.in_dll(capi.lib(), "fake_" + name)
+ctx = api.Context(0)
+def field(dims, loc=capi.CORNER, bc=capi.BC_DIRC, ext=0, ctx=ctx):
+    return api.CartesianField(cm.mesh_uniform(list(dims)), cm.field_desc(len(dims), loc, [(bc, bc)] * len(dims), ext=ext), ctx)
+""" % [ROOT, os.path.join(ROOT, "tests")]
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from opflow_gb300 import build
+    build.build()
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include")
+    out = str(tmp_path_factory.mktemp("fake") / "lib.so")
+    subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", inc, os.path.join(ROOT, "tests", "fake_cuda", "fake_cudart.cpp")] +
+                          sorted(glob.glob(os.path.join(build.BUILD, "*.o"))) + ["-o", out])
+    return out
+
+
+def _run(lib, code):
+    r = subprocess.run([sys.executable, "-c", HEAD + code, lib], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr[-2000:])
+
+
+def test_a_batch_with_fields_that_have_nothing_to_assign(fake):
+    # node-centred Dirichlet fields of two nodes along a direction: every node is a boundary node
+    _run(fake, """
+work = [(u, cm.ftcs_expr(u, 0.01, len(d))) for d in [(2, 8), (8, 2), (9, 9), (8, 2, 8), (2, 8, 8), (8, 8, 2), (9, 8, 7)] for u in [field(d)]]
+api.assign_batch(work, steps=2)
+""")
+
+
+def test_march_length_of_an_empty_box(tmp_path):
+    from opflow_gb300 import build
+    src = tmp_path / "t.cu"
+    src.write_text("""#include "stencil_exact.h"
+int main() {
+    for (int d = 0; d < 3; ++d)
+        for (int nd = 2; nd <= 3; ++nd)
+            for (int empty = 0; empty < 2; ++empty) {
+                opg::Box b;
+                for (int q = 0; q < nd; ++q) b.hi[q] = 9;
+                if (empty) b.hi[d] = b.lo[d];
+                const int m = opg::exact_march(b, nd, 152, empty ? 0. : 1.);
+                if (m < 4 || m > 32) return 1;
+            }
+    return 0;
+}
+""")
+    exe = str(tmp_path / "t")
+    subprocess.check_call([build._nvcc(), "-O0", "-std=c++17", "--expt-relaxed-constexpr", "-I", build.CSRC, str(src), "-o", exe] + build.ARCH)
+    assert subprocess.run([exe]).returncode == 0
