@@ -882,16 +882,16 @@ static __device__ __noinline__ double2 apply_chunk(const LvlDev& L, const Krylov
             if (js > 0) lo = *(p - n0);
             else if (L.per[1]) lo = p[(long long) (n1 - 1) * n0];
         }
+        const bool self = ND > 1 && n1 == 1 && L.per[1];  // the only row is its own upper neighbour (offset 0)
         // neighbours of the row at q: x and upper y (2D: loaded a row ahead)
         auto row = [&](const double* __restrict__ q, int j, double& w, double& e, double& hi) {
-            const bool hn = ND > 1 && (j < n1 - 1 || L.per[1]);
-            const long long on = j < n1 - 1 ? n0 : hn ? -(long long) (n1 - 1) * n0 : 0;  // (0 also where the only row is its own neighbour)
+            const long long on = j < n1 - 1 ? n0 : L.per[1] ? -(long long) (n1 - 1) * n0 : 0;
             w = q[ow];
             e = q[oe];
             hi = ND > 1 ? q[on] : 0.;
             w = hw ? w : 0.;
             e = he ? e : 0.;
-            hi = hn ? hi : 0.;
+            hi = on != 0 || self ? hi : 0.;
         };
         double cf[2 * ND + 1], w, e, hi;
         int yc = -1;
