@@ -529,6 +529,7 @@ int update_padding_assign(opflow_field f) {
 
 int update_padding_assign_many(opflow_ctx ctx, const opflow_field* fs, int n) {
     std::vector<PadJob> jobs;
+    std::vector<opflow_field> padded;  // by the launches below
     long long most = 0;
     for (int i = 0; i < n; ++i) {
         opflow_field f = fs[i];
@@ -541,8 +542,8 @@ int update_padding_assign_many(opflow_ctx ctx, const opflow_field* fs, int n) {
             f->bc_fresh[f->cur] = true;
         } else if (pad_job(f, data, zones, &J)) {
             jobs.push_back(J);
+            padded.push_back(f);
             most = std::max(most, J.L.start[J.L.n]);
-            f->bc_fresh[f->cur] = true;
         } else {
             OPG_TRY(update_padding_assign(f));
         }
@@ -561,6 +562,7 @@ int update_padding_assign_many(opflow_ctx ctx, const opflow_field* fs, int n) {
         rc = check_launch("pad_jobs_kernel");
     }
     dev_free(ctx, d);
+    for (size_t q = 0; q < padded.size() && rc == OPFLOW_OK; ++q) padded[q]->bc_fresh[padded[q]->cur] = true;
     if (rc == OPFLOW_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = fail(OPFLOW_E_CUDA, "padding update failed: %s", cudaGetErrorString(cudaGetLastError()));
     return rc;
 }

@@ -66,3 +66,30 @@ int main() {
     exe = str(tmp_path / "t")
     subprocess.check_call([build._nvcc(), "-O0", "-std=c++17", "--expt-relaxed-constexpr", "-I", build.CSRC, str(src), "-o", exe] + build.ARCH)
     assert subprocess.run([exe]).returncode == 0
+
+
+def test_a_failed_padding_leaves_the_field_to_be_padded(fake):
+    # every allocation of a batched assignment fails once; the next call pads all the same
+    _run(fake, """
+u, v = field((9, 9)), field((9, 9))
+failed = 0
+for n in range(1, 20):
+    u.upload(u.download(), update_padding=False)
+    count("fail_alloc").value = n
+    try:
+        api.assign_batch([(u, 2.0 * v)])
+    except capi.OpflowError as e:
+        assert e.code == capi.E_NOMEM
+        failed += 1
+    done = count("fail_alloc").value > 0
+    count("fail_alloc").value = 0
+    if done:
+        break
+    at = count("launches").value
+    api.assign_batch([(u, 2.0 * v)])
+    assert count("launches").value - at == 2, (n, count("launches").value - at)  # the assignment and the boundary nodes
+    at = count("launches").value
+    api.assign_batch([(u, 2.0 * v)])
+    assert count("launches").value - at == 1, n  # which hold their values now
+assert failed >= 2
+""")
