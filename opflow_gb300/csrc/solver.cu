@@ -628,6 +628,25 @@ static std::string level_key(const char* kernel, const MGSystem* S, int l) {
     return buf;
 }
 
+// The key of a level that mg_vol runs: apart from the z-marching kernels', whose values mean other things (a level of
+// the same extents may be theirs, where it is periodic).  A batch's holds the extents of all its fused levels.
+static std::string vol_key(const MGSystem* S, int l) {
+    std::string key = level_key("mg_smooth_z", S, l) + "/fused";
+    if (S->probs.size() > 1) {
+        unsigned long long h = tune_hash(nullptr, 0);
+        int last = -1;
+        for (const Chunk& t : S->vol_ch[l])
+            if (t.lvl != last) {
+                last = t.lvl;
+                h = tune_hash(S->lv_host[last].n, sizeof S->lv_host[last].n, h);
+            }
+        char buf[24];
+        std::snprintf(buf, sizeof buf, "/%016llx", h);
+        key += buf;
+    }
+    return key;
+}
+
 // The tuner's choices for a finalized system (tune.h): the plane batch of every z-marching level and,
 // on single-problem systems, the 2D tile shape of every tiled level, each timed on the level itself.
 // The level vectors are zeroed first; every V-cycle rewrites them before reading them.
@@ -681,7 +700,7 @@ static int tune_levels(MGSystem* S) {
                 }
                 return &e.second;
             };
-            const int pick = choose(level_key("mg_smooth_z", S, l), {4, 2, 8, MG_ZB_TMA}, [&](int c) {
+            const int pick = choose(vol_key(S, l), {4, 2, 8, 16}, [&](int c) {
                 const ChunkList* T = list(c);
                 if (!T) return -1.f;
                 return time_launch(S, [&] {

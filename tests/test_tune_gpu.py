@@ -152,3 +152,32 @@ def test_batch_level_mixing_row_lengths_keeps_every_problem_smoothed(ctx, fresh,
     assert got[0] == plain[0]
     for a, b in zip(got[1], plain[1]):
         assert np.array_equal(a, b)
+
+
+def test_fused_and_z_marching_levels_have_keys_of_their_own(ctx, fresh, tmp_path):
+    # levels of equal extents that different kernels run, and batches of equal cell totals
+    def keys(name, fn):
+        api.tune_clear()
+        api.tune_set_cache(tmp_path / name)
+        fn()
+        return {ln.split()[0] for ln in (tmp_path / name).read_text().splitlines()}
+    par = api.StructSolverParams(tol=1e-6, maxIter=20, precision="mixed")
+
+    def solve(n, bc):
+        fd = cm.field_desc(3, capi.CENTER, [(bc, bc)] * 3, ext=1)
+        u, f = (api.CartesianField(cm.mesh_uniform([m + 1 for m in n]), fd, ctx) for _ in range(2))
+        f.assign(1.0)
+        api.Solve(lambda e: f == e - 0.01 * (api.d2x(e) + api.d2y(e) + api.d2z(e)), u, par)
+
+    def batch(dims):
+        B = api.Batch([api.Problem(n, [1.0 / m for m in n], alpha=1.0, beta=0.01, loc=capi.CENTER, bc=capi.BC_NEUM) for n in dims], par, ctx)
+        for i in range(len(dims)):
+            B.set(i, np.ones(B.size(i)), np.zeros(B.size(i)))
+        B.solve()
+    sets = [keys("a", lambda: solve([128, 96, 96], capi.BC_NEUM)), keys("b", lambda: solve([128, 96, 96], capi.BC_PERIODIC)),
+            keys("c", lambda: batch([[64, 64, 48]] * 2)), keys("d", lambda: batch([[64, 64, 64], [64, 64, 32]])),
+            keys("e", lambda: batch([[64, 48, 64], [48, 64, 64]]))]
+    assert all(sets)
+    for i in range(len(sets)):
+        for j in range(i):
+            assert not sets[i] & sets[j], (i, j, sets[i] & sets[j])
