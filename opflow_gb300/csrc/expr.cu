@@ -1081,6 +1081,7 @@ static bool tape_of(const std::vector<Instr>& prog, const LeafViews& leaves, Tap
     std::vector<int> st;
     auto pop = [&] { const int v = st.back(); st.pop_back(); return v; };
     for (const Instr& in : prog) {
+        if (T->too_long()) return false;  // (every value of a stack program reaches its result)
         switch (in.op) {
             case P_LOAD: st.push_back(T->load(in.slot, leaves.v[in.slot], in.off)); break;
             case P_CONST: st.push_back(T->cst(in.v)); break;

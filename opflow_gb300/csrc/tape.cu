@@ -43,8 +43,10 @@ int Tape::intern(const Node& n) {
     auto it = index_.find(key);
     if (it != index_.end()) return it->second;
     nodes_.push_back(n);
+    per_cell_ += n.op != T_CONST && n.op != T_NEG && n.dep != 1 && n.dep != 2 && n.dep != 4;
     return index_[key] = (int) nodes_.size() - 1;
 }
+bool Tape::too_long() const { return per_cell_ > TP_CODE; }
 
 int Tape::cst(double v) { return intern(Node{T_CONST, 0, -1, -1, -1, 0, v, 0}); }
 int Tape::load(int slot, const FieldView& f, const int* off) {

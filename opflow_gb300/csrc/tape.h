@@ -56,6 +56,9 @@ public:
     int node(int op, int slot, int a, int b = -1, int c = -1);
     bool is_const(int id, double* v) const;
     void out(int op, int slot, int id) { outs_.push_back({op, slot, id}); }
+    // Whether the values formed so far, each of them read by the program's result, are already more than the kernel
+    // takes (constants, negations and values of one direction left out: they may go elsewhere); finish() is then false.
+    bool too_long() const;
     // Lays the program out; `hoist`: values of one direction go to tables.  false: too long, or too many values
     // live at once, for the kernel.
     bool finish(const Box& box, bool hoist);
@@ -80,6 +83,7 @@ private:
     Program main_, table_[3];
     std::vector<long long> tab_first_;  // per value: first table entry, -1 none
     long long tab_entries_ = 0;
+    int per_cell_ = 0;                  // values that only the cells' own program can form
     char* blob_ = nullptr;
     size_t off_tab_ = 0;
 };

@@ -93,3 +93,46 @@ for n in range(1, 20):
     assert count("launches").value - at == 1, n  # which hold their values now
 assert failed >= 2
 """)
+
+
+def test_programs_given_up_early_are_those_that_do_not_fit(fake, tmp_path):
+    # around the kernel's limit, of loads, constants, negations, quotients and values of one direction
+    from opflow_gb300 import build
+    src, exe = tmp_path / "t.cpp", str(tmp_path / "t")
+    src.write_text("""#include "tape.h"
+#include <cstdio>
+using namespace opg;
+int main() {
+    int early = 0, fit = 0;
+    for (int n = 100; n <= 900; n += 7)
+        for (int kind = 0; kind < 4; ++kind)
+            for (int hoist = 0; hoist < 2; ++hoist) {
+                Tape T;
+                FieldView f{};
+                f.sy = 100;
+                f.sz = 10000;
+                int v = T.cst(0.5);
+                bool gave_up = false;
+                for (int q = 0; q < n; ++q) {
+                    const int off[3] = {q % 90, q / 90, 0};
+                    int t = kind == 1 ? T.bin(T_MUL, T.pos(T_X, q & 1, q % 5), T.cst(1. + q)) : T.load(0, f, off);
+                    if (kind == 2) t = T.neg(t);
+                    if (kind == 3) t = T.bin(T_DIV, t, T.bin(T_ADD, T.pos(T_X, 0, 0), T.cst(q)));
+                    v = T.bin(q % 3 ? T_ADD : T_SUB, v, t);
+                    gave_up = gave_up || T.too_long();
+                }
+                T.out(T_OUT, 0, v);
+                Box b;
+                b.hi[0] = b.hi[1] = 50;
+                const bool ok = T.finish(b, hoist);
+                if (gave_up && ok) return printf("%d values of kind %d\\n", n, kind), 1;
+                early += gave_up;
+                fit += ok;
+            }
+    return early > 0 && fit > 0 ? 0 : 2;
+}
+""")
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", build.CSRC, "-I", inc, str(src), fake, "-o", exe])
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stdout)
