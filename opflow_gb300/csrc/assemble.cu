@@ -586,13 +586,16 @@ static void plain_rhs(const std::vector<PInstr>& prog, AsmPlan* plan) {
 
 // The inner cells' coefficients and right-hand side as a scalar program: there every leaf of the unknown is one
 // coefficient 1 and no bias, so a pad's entries are values or absent, and only the present ones are formed
-// (the reference's StencilPad holds no others either).  coef: with the coefficients, else the right-hand side
-// alone.
+// (the reference's StencilPad holds no others either).  Its bias is always there, a zero at the leaves: it stays one
+// but where a factor is infinite or NaN, which makes it NaN.  So the factors of all pads are kept, and the
+// right-hand side is NaN where one of them is not finite (integer operations; those of one direction in a table).
+// coef: with the coefficients, else the right-hand side alone.
 static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
     const AsmParams& P = plan.P;
     struct Pad { std::map<int, int> c; int b = -1; };  // entry -> value, bias value (-1: none)
     std::vector<Pad> pads;
     std::vector<int> nums;
+    std::set<int> factors;
     auto num = [&] { const int v = nums.back(); nums.pop_back(); return v; };
     for (const PInstr& in : plan.prog) {
         switch (in.op) {
@@ -655,6 +658,7 @@ static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
                 } else {
                     // a product with a number, or pad / num = pad * (1. / num)
                     const int s = op == T_DIV ? T->bin(T_DIV, T->cst(1.0), B.b) : in.ta ? B.b : A.b;
+                    factors.insert(s);
                     if (!in.ta) A = B;
                     for (auto& e : A.c) e.second = T->bin(T_MUL, e.second, s);
                     if (A.b >= 0) A.b = T->bin(T_MUL, A.b, s);
@@ -666,7 +670,18 @@ static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
     const Pad& r = pads.back();
     if (coef)
         for (int q = 0; q < P.nk; ++q) T->out(T_COEF, q, r.c.count(q) ? r.c.at(q) : T->cst(0.0));
-    T->out(T_RHS, 0, r.b >= 0 ? T->neg(r.b) : T->cst(0.0));
+    int rhs = r.b >= 0 ? T->neg(r.b) : T->cst(0.0), of_dir[3];
+    for (int d = 0; d < 3; ++d) of_dir[d] = T->cst(0.0);
+    for (int s : factors) {
+        double v;
+        if (T->is_const(s, &v) && std::isfinite(v)) continue;
+        const int d = T->direction(s);
+        int& z = d >= 0 ? of_dir[d] : rhs;
+        z = T->node(T_FIN, 0, z, s);
+    }
+    for (int d = 0; d < 3; ++d)
+        if (T->direction(of_dir[d]) == d) rhs = T->node(T_FIN, 0, rhs, of_dir[d]);
+    T->out(T_RHS, 0, rhs);
     return true;
 }
 

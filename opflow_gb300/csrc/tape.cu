@@ -60,6 +60,11 @@ bool Tape::is_const(int id, double* v) const {
     return true;
 }
 
+int Tape::direction(int id) const {
+    const int d = nodes_[id].dep;
+    return d == 1 ? 0 : d == 2 ? 1 : d == 4 ? 2 : -1;
+}
+
 int Tape::node(int op, int slot, int a, int b, int c) {
     Node n{op, slot, a, b, c, 0, 0., 0};
     for (int q : {a, b, c})
@@ -183,7 +188,7 @@ bool Tape::emit(const std::vector<Out>& outs, const std::vector<int>& tab, Progr
         if (tab[s.id]) {
             in.op = T_TAB;
             in.lin = tab_first_[s.id];
-            in.slot = n.dep == 1 ? 0 : n.dep == 2 ? 1 : 2;
+            in.slot = direction(s.id);
         } else {
             in.a = operand(n.a);
             in.b = operand(n.b);
@@ -221,17 +226,16 @@ bool Tape::finish(const Box& box, bool hoist) {
     if (hoist) {
         std::vector<int> need(nodes_.size(), 0);
         for (const Out& o : outs_) need[o.id] = 1, root[o.id] = 1;
-        auto one_dir = [&](int id) { const int d = nodes_[id].dep; return d == 1 || d == 2 || d == 4; };
         for (int id = (int) nodes_.size() - 1; id >= 0; --id) {
             if (!need[id]) continue;
             const Node& n = nodes_[id];
-            if (one_dir(id) && n.op != T_X && n.op != T_DX) { tab[id] = 1; continue; }
+            if (direction(id) >= 0 && n.op != T_X && n.op != T_DX) { tab[id] = 1; continue; }
             for (int q : {n.a, n.b, n.c})
                 if (q >= 0) need[q] = 1;
         }
         for (int id = 0; id < (int) nodes_.size(); ++id)
             if (tab[id]) {
-                const int d = nodes_[id].dep == 1 ? 0 : nodes_[id].dep == 2 ? 1 : 2;
+                const int d = direction(id);
                 tab_first_[id] = tab_entries_;
                 tab_entries_ += box.hi[d] - box.lo[d];
                 touts[d].push_back({T_TABOUT, d, id});
@@ -341,6 +345,7 @@ __global__ void __launch_bounds__(TP_THREADS) tape_kernel(const __grid_constant_
                 case T_OR: EACH_CELL r[c] = get(in.a, c) != 0. || get(in.b, c) != 0. ? 1. : 0.; break;
                 case T_NOT: EACH_CELL r[c] = get(in.a, c) == 0. ? 1. : 0.; break;
                 case T_SEL: EACH_CELL r[c] = get(in.a, c) != 0. ? get(in.b, c) : get(in.c, c); break;
+                case T_FIN: EACH_CELL r[c] = (__double2hiint(get(in.b, c)) & 0x7FF00000) == 0x7FF00000 ? __longlong_as_double(0x7FF8000000000000ll) : get(in.a, c); break;
                 case T_F1: EACH_CELL r[c] = func1_eval(in.slot, get(in.a, c)); break;
                 case T_F2: EACH_CELL r[c] = func2_eval(in.slot, get(in.a, c), get(in.b, c)); break;
                 case T_LIM: EACH_CELL r[c] = flux_limiter(in.slot, get(in.a, c)); break;

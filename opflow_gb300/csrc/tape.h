@@ -18,6 +18,7 @@ enum TOp : int {
     T_RCP, T_NEG,
     T_GT, T_GE, T_LT, T_LE, T_NE, T_AND, T_OR, T_NOT, T_SEL,  // (T_SEL: a ? b : c)
     T_F1, T_F2, T_LIM,
+    T_FIN,                       // a where b is finite, else NaN
     T_TAB,                       // a tabulated value of one direction
     T_OUT, T_COEF, T_RHS, T_TABOUT
 };
@@ -55,6 +56,7 @@ public:
     int neg(int a);
     int node(int op, int slot, int a, int b = -1, int c = -1);
     bool is_const(int id, double* v) const;
+    int direction(int id) const;  // the direction whose mesh positions alone a value depends on, -1: none or several
     void out(int op, int slot, int id) { outs_.push_back({op, slot, id}); }
     // Whether the values formed so far, each of them read by the program's result, are already more than the kernel
     // takes (constants, negations and values of one direction left out: they may go elsewhere); finish() is then false.

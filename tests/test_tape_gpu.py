@@ -131,3 +131,36 @@ def test_assembled_inner_cells_match_the_oracle(ctx, n, stretched, bc, pin):
     for q, o in enumerate(want_off.tolist()):
         assert np.array_equal(got[tuple(o)], want_coef[:, q]), (o, np.abs(got[tuple(o)] - want_coef[:, q]).max())
     assert np.array_equal(rhs, want_rhs)
+
+
+@pytest.mark.parametrize("n", [[80, 70], [40, 33, 20]])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_infinite_and_nan_coefficients_reach_the_right_hand_side(ctx, n, bad):
+    # the bias of a pad is always there, and 0 times an infinite factor is NaN
+    D = len(n)
+    mesh = cm.mesh_uniform([m + 1 for m in n])
+    fd = cm.field_desc(D, capi.CENTER, [(capi.BC_DIRC, capi.BC_DIRC)] * D, [(0.3, -0.2)] * D, ext=1)
+    rng = np.random.default_rng(sum(n))
+    hosts = [orc.HostField(mesh, fd) for _ in range(3)]
+    for h in hosts[1:]:
+        sl = h.slices(h.assignable())
+        v = rng.random(h.data[sl].shape) + 0.5
+        if h is hosts[1]:
+            v.flat[rng.integers(0, v.size, 40)] = bad
+        h.data[sl] = v
+        h.update_padding()
+    dev = [api.CartesianField(mesh, fd, ctx) for _ in hosts]
+    for a, h in zip(dev, hosts):
+        a.upload(h.data, update_padding=False)
+
+    def eq(p, K, f):
+        t = 2.0 * p
+        for d in range(D):
+            t = t - api.d1(api.d1IntpCenterToCorner(K, d) * api.d1(p, d), d)
+        return api.Eq(t, f)
+    L = [cm.Leaf(x) for x in "pKf"]
+    nodes = api.serialize(eq(*L).residual_expr(), L)[0]
+    want = orc.assemble(hosts[0], nodes, hosts, 0, 0)[2]
+    rhs = api.assemble(lambda e: eq(e, dev[1], dev[2]), dev[0])[2]
+    assert np.isnan(want).any() and not np.isnan(want).all()
+    assert np.array_equal(rhs, want, equal_nan=True)
