@@ -15,11 +15,12 @@
 //  - x / 3, x / 6 and x / h are two operations, fma(x, c, x * c') with c + c' = 1/3, 1/6, 1/h to 106 bits,
 //    which is the correctly rounded quotient (div2_failures in stencil.cu: for 3 and 6 no significand can
 //    fail, for h the one that may is guarded); a power of two h moves the exponent field;
-//  - exact multiplications (by 2, 4, 1/4, and d / 6 = (d / 3) / 2) are folded into fused operations;
+//  - exact multiplications (by 2, 4, 1/4, and d / 6 = (d / 3) / 2) are folded into fused operations, apart where a
+//    result below the normal range makes them inexact;
 //  - the six IEEE divisions per point are built from four reciprocals (div_rn: the three weights share
 //    their denominator).
 // 84 float64 operations per point and stage against 119 with the reference's operations one by one:
-// 16384 lines of 4096 cells 44.2 -> 35.2 ms.
+// 16384 lines of 4096 cells 44.2 -> 35.3 ms.
 // FAST mode (not bit-identical) contracts the arithmetic and forms the three nonlinear weights with one
 // reciprocal.
 #include "f64div.h"
@@ -55,6 +56,17 @@ __device__ __forceinline__ bool out_of_range(double x) {
     const int hi = __double2hiint(x);
     return (unsigned) (((hi >> 20) & 0x7FF) - 150) > 1700u && ((hi & 0x7FFFFFFF) | __double2loint(x)) != 0;
 }
+
+// Whether 2^-k x is rounded: x below 2^(k - 1022), not zero.
+__device__ __forceinline__ bool rounds(double x, int k) {
+    const unsigned m = ((unsigned) __double2hiint(x) & 0x7FFFFFFFu) | (__double2loint(x) != 0);
+    return m - 1u < ((unsigned) (k + 1) << 20) - 1u;
+}
+// a / 4 + b in two roundings
+static __device__ __noinline__ double weno_quarter(double a, double b) { return __dadd_rn(__dmul_rn(0.25, a), b); }
+// (-d1 / 6 + b) + c and a - d4 / 6 with the quotients rounded
+static __device__ __noinline__ double weno_sixth2(double d1, double b, double c) { return __dadd_rn(__dadd_rn(-__ddiv_rn(d1, 6.), b), c); }
+static __device__ __noinline__ double weno_sixth3(double a, double d4) { return __dsub_rn(a, __ddiv_rn(d4, 6.)); }
 
 // correctly rounded x / c for the c whose reciprocal is ch + cl, x in range
 __device__ __forceinline__ double div_const(double x, double ch, double cl) { return __fma_rn(x, ch, __dmul_rn(x, cl)); }
@@ -132,10 +144,13 @@ __device__ __forceinline__ double weno_point(const DiffTerms& X0, const DiffTerm
     long long mb = max_bits(max_bits(max_bits(X0.SQ, X1.SQ), max_bits(X2.SQ, X3.SQ)), X4.SQ);
     const double mx = __longlong_as_double(mb);
     if constexpr (!FAST) {
-        // (d / 6 = (d / 3) / 2, 4 d and t / 4 are exact: folded into the operation that takes them)
+        // (d / 6 = (d / 3) / 2, 4 d and t / 4 are exact, d / 6 but for the smallest: folded into the operation that takes
+        // them; a t * t / 4 that is not vanishes beside eps)
         const double ddx1 = __dadd_rn(__dsub_rn(X0.D3, X1.D76), X2.D116);
-        const double ddx2 = __dadd_rn(__fma_rn(-0.5, X1.D3, X2.D56), X3.D3);
-        const double ddx3 = __fma_rn(-0.5, X4.D3, __dadd_rn(X2.D3, X3.D56));
+        double ddx2 = __dadd_rn(__fma_rn(-0.5, X1.D3, X2.D56), X3.D3);
+        double ddx3 = __fma_rn(-0.5, X4.D3, __dadd_rn(X2.D3, X3.D56));
+        if (rounds(X1.D3, 1)) ddx2 = weno_sixth2(X1.D, X2.D56, X3.D3);
+        if (rounds(X4.D3, 1)) ddx3 = weno_sixth3(__dadd_rn(X2.D3, X3.D56), X4.D);
         double t2 = __dadd_rn(__fma_rn(-4., X1.D, X0.D), X2.M3);
         const double s1 = __fma_rn(0.25, __dmul_rn(t2, t2), p0);
         t2 = __dsub_rn(X1.D, X3.D);
@@ -227,7 +242,11 @@ __device__ __forceinline__ void weno_stage(const double* __restrict__ u, const d
             const double L = FAST ? r : __dmul_rn(P.dt, r);
             double v;
             if constexpr (STAGE == 0) v = __dsub_rn(u[i], L);
-            else if constexpr (STAGE == 1) v = __fma_rn(0.25, __dsub_rn(src[i], L), __dmul_rn(0.75, u[i]));  // (x / 4 is exact)
+            else if constexpr (STAGE == 1) {
+                const double w = __dsub_rn(src[i], L), z = __dmul_rn(0.75, u[i]);
+                v = __fma_rn(0.25, w, z);  // (w / 4 is exact but for the smallest)
+                if (!FAST && rounds(w, 2)) v = weno_quarter(w, z);
+            }
             else v = __dadd_rn(__dmul_rn(P.third, u[i]), __dmul_rn(P.two_third, __dsub_rn(src[i], L)));
             out[i] = v;
             X[0] = X[1];

@@ -2,6 +2,8 @@
 lengths around a thread's points, power-of-two and other spacings (1/300 leaves one significand out of the
 two-operation division), both sides, and values that reach every branch: smooth, jumps, constants, zeros,
 and magnitudes over most of the exponent range."""
+import sys
+
 import numpy as np
 import pytest
 
@@ -45,3 +47,12 @@ def test_fused_weno_matches_the_oracle(ctx, n, upwind):
                 orc.assign(dst, nd, h)
         got, want = u.download()[sl], h[0].data[sl]
         assert np.array_equal(got, want, equal_nan=True), (name, np.abs(got - want).max())
+
+
+@pytest.mark.parametrize("n", [17, 97, 300])
+@pytest.mark.parametrize("upwind", [False, True])
+@pytest.mark.parametrize("low,high", [(-1074, -1000), (-1074, -1040), (-1060, -900)])
+def test_fused_weno_below_the_normal_range(ctx, monkeypatch, n, upwind, low, high):
+    values = lambda r, s: r.standard_normal(s) * 2.0 ** r.integers(low, low + 30, s) * 2.0 ** r.integers(0, high - low - 29, s)
+    monkeypatch.setattr(sys.modules[__name__], "VALUES", {"subnormal": values})
+    test_fused_weno_matches_the_oracle(ctx, n, upwind)
