@@ -23,6 +23,8 @@ struct LvlDev {
     int table;           // 1: coefficients from the class table, 0: SoA arrays
     int uoff;            // 1 (class tables): every off-diagonal coefficient of an existing neighbour equals the
                          // interior class's, so the classes differ in the centre one only
+    int adjoint;         // cell-centred restriction into the next level: 0 averages over the children that exist, 1 sums
+                         // them with the weight of a whole cell's (the interpolation's adjoint, see ProblemHost::adjoint)
     int rbgs;            // 1: red-black Gauss-Seidel, 0: damped Jacobi
     int problem;         // owning problem
     int coarsest;        // 1 if no coarser level

@@ -169,7 +169,7 @@ __device__ __forceinline__ void cell_restrict(const LvlDev* __restrict__ Ls, con
     const long long cc = cell_of(Lc, I[0], I[1], I[2]);
     T acc = 0;
     if (!Lc.node) {
-        // average of the children that exist
+        // average of the children that exist, or their sum with the same weights everywhere
         int cnt = 0;
         for (int dz = 0; dz < (Lc.ndim > 2 ? 2 : 1); ++dz)
             for (int dy = 0; dy < (Lc.ndim > 1 ? 2 : 1); ++dy)
@@ -180,7 +180,7 @@ __device__ __forceinline__ void cell_restrict(const LvlDev* __restrict__ Ls, con
                         cnt++;
                     }
                 }
-        acc = acc / (T) cnt;
+        acc = Lf.adjoint ? acc * (Lc.ndim > 2 ? (T) 0.125 : Lc.ndim > 1 ? (T) 0.25 : (T) 0.5) : acc / (T) cnt;
     } else {
         // full weighting on absolute node indices: coarse node I <-> fine node 2I
         const int ga[3] = {Lc.lo[0] + I[0], Lc.lo[1] + I[1], Lc.lo[2] + I[2]};

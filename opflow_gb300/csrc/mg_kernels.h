@@ -68,6 +68,7 @@ struct SmLevel {
     int s1, s2;          // strides of rows and planes (cells, the ring of zeros included)
     int x, b;            // places of cell (0, 0, 0)
     int node;            // node-centred transfers to this level from the next finer one
+    int adjoint;         // LvlDev::adjoint
     int barrier;         // the level's named barrier
     int lw;                        // a warp share: 2^lw column pairs of 32 / 2^lw rows
     int half, pairs, shares;       // shares along a row, along the rows of a plane, in all
@@ -87,7 +88,7 @@ struct SmProblem {
     SmLevel lv[MG_BOTTOM_LEVELS];
 };
 struct SmSource {  // one level as mg_small_problem takes it
-    int ndim, n[3], lo[3], per[3], glo[3], ghi[3], node;
+    int ndim, n[3], lo[3], per[3], glo[3], ghi[3], node, adjoint;
     const std::vector<double>* tab;  // class table, NSLOT per class
 };
 bool mg_small_problem(const SmSource* L, int levels, const double* Ainv, SmProblem* P, long long* floats);

@@ -139,7 +139,7 @@ struct Small {
         float* bc = sm + Lc.b;
         const int nc0 = Lc.n[0], nc1 = Lc.n[1];
         if (!Lc.node) {
-            // the average of the children that exist (warps take 2^lf cells of 32 / 2^lf rows)
+            // the average of the children that exist, or with all's weight (warps take 2^lf cells of 32 / 2^lf rows)
             const int lf = Lc.lf, groups = Lc.fgroups, rows = Lc.frows, total = groups * rows * (ND > 2 ? Lc.n[2] : 1);
             for (int g = warp; g < total; g += act) {
                 const int rg = groups == 1 ? g : g / groups, K = ND > 2 ? small_div(rg, Lc.mfrows) : 0;
@@ -155,7 +155,7 @@ struct Small {
                         ++n;
                     }
                 }
-                bc[I + J * Lc.s1 + (ND > 2 ? K * Lc.s2 : 0)] = __fmul_rn(acc, n == 8 ? 0.125f : n == 4 ? 0.25f : n == 2 ? 0.5f : 1.f);
+                bc[I + J * Lc.s1 + (ND > 2 ? K * Lc.s2 : 0)] = __fmul_rn(acc, L.adjoint ? (ND > 2 ? 0.125f : 0.25f) : n == 8 ? 0.125f : n == 4 ? 0.25f : n == 2 ? 0.5f : 1.f);
             }
         } else {
 #pragma unroll 1
@@ -369,6 +369,7 @@ bool mg_small_problem(const SmSource* L, int levels, const double* Ainv, SmProbl
         if (frames > MG_SMALL_FLOATS) return false;
         D.barrier = 1 + q;
         D.node = S.node;
+        D.adjoint = S.adjoint;
         P->node |= S.node;
         auto magic = [](unsigned d) { return 0xFFFFFFFFu / d + 1; };  // (d = 1: 0)
         const int hw = (D.n[0] + 1) / 2;

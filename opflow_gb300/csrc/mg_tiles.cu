@@ -231,8 +231,8 @@ __device__ __forceinline__ void strip_down(const LvlDev& L, const LvlDev& Lc, co
             if (P == 0) {
                 pa = __fadd_rn(re, ro);
             } else if (own_e && r - 1 >= S.j0 && r - 1 < S.j1) {
-                // average over the children that exist: 4, 2 or 1
-                const float sc = (r < S.n1 ? 0.5f : 1.f) * (oin ? 0.5f : 1.f);
+                // average over the children that exist: 4, 2 or 1 (adjoint: as if all did)
+                const float sc = (r < S.n1 || L.adjoint ? 0.5f : 1.f) * (oin || L.adjoint ? 0.5f : 1.f);
                 const long long cc = (long long) (r >> 1) * cn0 + (S.ge >> 1);
                 bc[cc] = __fmul_rn(__fadd_rn(__fadd_rn(pa, re), ro), sc);
                 xc[cc] = 0.f;

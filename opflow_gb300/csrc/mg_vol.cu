@@ -223,8 +223,8 @@ __device__ __forceinline__ void vol_down(const LvlDev& L, const LvlDev& Lc, cons
         } else {
             const float acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(pa, res[0][0]), res[0][1]), res[1][0]), res[1][1]);
             if (own_e && own_r[0] && p - 1 >= T.k0 && p - 1 < T.k1) {
-                // average over the children that exist: 8, 4, 2 or 1
-                const float sc = (p < T.n2 ? 0.5f : 1.f) * (T.okr[1] ? 0.5f : 1.f) * (T.oko ? 0.5f : 1.f);
+                // average over the children that exist: 8, 4, 2 or 1 (adjoint: as if all did)
+                const float sc = L.adjoint ? 0.125f : (p < T.n2 ? 0.5f : 1.f) * (T.okr[1] ? 0.5f : 1.f) * (T.oko ? 0.5f : 1.f);
                 const long long cc = (T.ge >> 1) + (long long) Lc.n[0] * ((T.y0 >> 1) + (long long) Lc.n[1] * (p >> 1));
                 Lc.b32[cc] = __fmul_rn(acc, sc);
                 Lc.x32[cc] = 0.f;

@@ -568,6 +568,8 @@ int mg_add_problem(MGSystem* S, opflow_field target, const opflow_node* nodes, i
         cur_target = ct;
         cur_leaves = nl;
     }
+    for (size_t l = 0; l + 1 < P.levels.size() && P.singular && !P.has_dirichlet; ++l)
+        for (int d = 0; d < P.levels[l].ndim; ++d) P.adjoint = P.adjoint || ((P.levels[l].n[d] & 1) && P.levels[l].n[d] > ADJOINT_FROM);
     for (auto& L : P.levels) OPG_TRY(compress_level(S, L));
     // coarsest: direct solve when small enough, else smoothing only
     LevelHost& Lc = P.levels.back();
@@ -889,6 +891,7 @@ int mg_finalize(MGSystem* S) {
                     X.ghi[d] = H.gh_hi[d];
                 }
                 X.node = H.node;
+                X.adjoint = P.adjoint;
                 X.tab = &H.tab;
                 src.push_back(X);
             }
@@ -933,6 +936,7 @@ int mg_finalize(MGSystem* S) {
             D.node = H.node;
             D.table = H.table;
             D.uoff = H.uoff;
+            D.adjoint = P.adjoint;
             bool odd_periodic = false;
             for (int d = 0; d < H.ndim; ++d) odd_periodic = odd_periodic || (H.per[d] && (H.n[d] & 1));
             D.rbgs = !odd_periodic;
