@@ -589,8 +589,10 @@ static void plain_rhs(const std::vector<PInstr>& prog, AsmPlan* plan) {
 // (the reference's StencilPad holds no others either).  Its bias is always there, a zero at the leaves: it stays one
 // but where a factor is infinite or NaN, which makes it NaN.  So the factors of all pads are kept, and the
 // right-hand side is NaN where one of them is not finite (integer operations; those of one direction in a table).
-// coef: with the coefficients, else the right-hand side alone.
-static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
+// coef: with the coefficients, else the right-hand side alone, for a kept matrix; factors of fields that have not been
+// written since (AsmPlan::as_assembled) are not formed again then: where one is not finite, the matrix is not
+// either.  hoist: as for Tape::finish.
+static bool inner_tape(const AsmPlan& plan, bool coef, bool hoist, Tape* T) {
     const AsmParams& P = plan.P;
     struct Pad { std::map<int, int> c; int b = -1; };  // entry -> value, bias value (-1: none)
     std::vector<Pad> pads;
@@ -668,17 +670,33 @@ static bool inner_tape(const AsmPlan& plan, bool coef, Tape* T) {
         }
     }
     const Pad& r = pads.back();
-    if (coef)
-        for (int q = 0; q < P.nk; ++q) T->out(T_COEF, q, r.c.count(q) ? r.c.at(q) : T->cst(0.0));
     int rhs = r.b >= 0 ? T->neg(r.b) : T->cst(0.0), of_dir[3];
     for (int d = 0; d < 3; ++d) of_dir[d] = T->cst(0.0);
+    std::vector<int> left;  // factors formed per cell
     for (int s : factors) {
         double v;
         if (T->is_const(s, &v) && std::isfinite(v)) continue;
-        const int d = T->direction(s);
-        int& z = d >= 0 ? of_dir[d] : rhs;
-        z = T->node(T_FIN, 0, z, s);
+        if (!coef && (T->fields(s) & ~plan.as_assembled) == 0) continue;
+        const int d = hoist ? T->direction(s) : -1;
+        if (d >= 0) of_dir[d] = T->node(T_FIN, 0, of_dir[d], s);
+        else left.push_back(s);
     }
+    auto look_at = [&](int s) {
+        rhs = T->node(T_FIN, 0, rhs, s);
+        T->form(rhs);
+    };
+    if (coef)
+        for (int q = 0; q < P.nk; ++q) {
+            const int c = r.c.count(q) ? r.c.at(q) : T->cst(0.0);
+            T->out(T_COEF, q, c);
+            // (a factor is looked at beside the first coefficient it goes into: none is kept longer for it)
+            for (size_t k = 0; k < left.size();) {
+                if (!T->uses(c, left[k])) { ++k; continue; }
+                look_at(left[k]);
+                left.erase(left.begin() + k);
+            }
+        }
+    for (int s : left) look_at(s);
     for (int d = 0; d < 3; ++d)
         if (T->direction(of_dir[d]) == d) rhs = T->node(T_FIN, 0, rhs, of_dir[d]);
     T->out(T_RHS, 0, rhs);
@@ -906,7 +924,8 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
     const bool plain = !coef && plan->rhs_plain && !plan->P.pin && !in.empty();
     Tape tape;
     bool taped = false;
-    if (!plain && !pinned && in.count() >= ASM_TAPE_CELLS) taped = inner_tape(*plan, coef != nullptr, &tape) && tape.finish(in, in.count() >= 32768);
+    const bool hoist = in.count() >= 32768;
+    if (!plain && !pinned && in.count() >= ASM_TAPE_CELLS) taped = inner_tape(*plan, coef != nullptr, hoist, &tape) && tape.finish(in, hoist);
     int rc = OPFLOW_OK;
     if (plain) {
         const int nx = in.hi[0] - in.lo[0], rows = (in.hi[1] - in.lo[1]) * (in.hi[2] - in.lo[2]);

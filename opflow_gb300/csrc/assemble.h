@@ -53,6 +53,7 @@ struct AsmPlan {
     int rhs_slot = 0, rhs_off[3] = {0, 0, 0};
     double rhs_sign = 0.;
     Box inner;
+    unsigned as_assembled = 0;  // for a right-hand side alone: bit k: leaf k is unwritten since the matrix was assembled
     std::vector<PInstr> prog;
     std::vector<std::array<int, 3>> comm;  // middle cell's stencil keys, offset form, insertion order
     long long cells = 0;

@@ -1673,7 +1673,7 @@ struct opflow_solver_s {
     MGSystem* S = nullptr;
     bool first = true;
     // write counters of the leaves when the system was last assembled (the target's after its solve)
-    std::vector<unsigned long long> assembled_versions;
+    std::vector<unsigned long long> assembled_versions, matrix_versions;  // (matrix: of the kept matrix's assembly)
     // generateb's compiled plan (staticMat), made on the first re-solve
     AsmPlan rhs_plan;
     bool rhs_plan_ok = false;
@@ -1687,6 +1687,7 @@ static std::vector<unsigned long long> leaf_versions(opflow_solver s) {
 }
 
 static int build_system(opflow_solver s) {
+    s->matrix_versions = leaf_versions(s);
     if (s->S) mg_destroy(s->S);
     s->S = new MGSystem();
     s->S->ctx = s->ctx;
@@ -1771,7 +1772,12 @@ int opflow_solver_solve(opflow_solver s, opflow_solve_state* state) {
                                     &s->rhs_plan));
                 s->rhs_plan_ok = true;
             }
-            for (size_t k = 0; k < s->leaves.size(); ++k) s->rhs_plan.P.leaves[k] = s->leaves[k]->view();
+            s->rhs_plan.as_assembled = 0;
+            const std::vector<unsigned long long> now = leaf_versions(s);
+            for (size_t k = 0; k < s->leaves.size(); ++k) {
+                s->rhs_plan.P.leaves[k] = s->leaves[k]->view();
+                if (now[k] == s->matrix_versions[k]) s->rhs_plan.as_assembled |= 1u << k;
+            }
             OPG_TRY(asm_run(ctx, &s->rhs_plan, nullptr, s->S->probs[0].b));
         } else {
             OPG_TRY(build_system(s));

@@ -65,6 +65,29 @@ int Tape::direction(int id) const {
     return d == 1 ? 0 : d == 2 ? 1 : d == 4 ? 2 : -1;
 }
 
+bool Tape::uses(int id, int operand) const {
+    if (id < operand) return false;  // (operands come first)
+    std::vector<char> from(id + 1 - operand, 0);
+    from[0] = 1;
+    for (int q = operand + 1; q <= id; ++q)
+        for (int o : {nodes_[q].a, nodes_[q].b, nodes_[q].c})
+            if (o >= operand && from[o - operand]) from[q - operand] = 1;
+    return from[id - operand];
+}
+
+unsigned Tape::fields(int id) const {
+    std::vector<char> in(id + 1, 0);
+    in[id] = 1;
+    unsigned f = 0;
+    for (int q = id; q >= 0; --q) {
+        if (!in[q]) continue;
+        if (nodes_[q].op == T_LOAD) f |= 1u << nodes_[q].slot;
+        for (int o : {nodes_[q].a, nodes_[q].b, nodes_[q].c})
+            if (o >= 0) in[o] = 1;
+    }
+    return f;
+}
+
 int Tape::node(int op, int slot, int a, int b, int c) {
     Node n{op, slot, a, b, c, 0, 0., 0};
     for (int q : {a, b, c})
@@ -151,7 +174,7 @@ bool Tape::emit(const std::vector<Out>& outs, const std::vector<int>& tab, Progr
         order.clear();
         visit(o.id);
         for (int id : order) steps.push_back({id, {}});
-        steps.push_back({-1, o});
+        if (o.op != T_CONST) steps.push_back({-1, o});
     }
     for (const Step& s : steps) {
         if (s.id < 0) { ++uses[s.out.id]; continue; }

@@ -58,6 +58,9 @@ public:
     bool is_const(int id, double* v) const;
     int direction(int id) const;  // the direction whose mesh positions alone a value depends on, -1: none or several
     void out(int op, int slot, int id) { outs_.push_back({op, slot, id}); }
+    void form(int id) { outs_.push_back({T_CONST, 0, id}); }  // here in the program, read by a later one
+    bool uses(int id, int operand) const;                     // whether id is, or is formed from, operand
+    unsigned fields(int id) const;                            // the leaf slots that id is formed from, a bit each
     // Whether the values formed so far, each of them read by the program's result, are already more than the kernel
     // takes (constants, negations and values of one direction left out: they may go elsewhere); finish() is then false.
     bool too_long() const;

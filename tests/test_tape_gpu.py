@@ -164,3 +164,29 @@ def test_infinite_and_nan_coefficients_reach_the_right_hand_side(ctx, n, bad):
     rhs = api.assemble(lambda e: eq(e, dev[1], dev[2]), dev[0])[2]
     assert np.isnan(want).any() and not np.isnan(want).all()
     assert np.array_equal(rhs, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [[80, 70], [40, 33, 20]])
+def test_coefficients_that_become_infinite_reach_a_kept_matrix_s_right_hand_side(ctx, n):
+    # staticMat: the right-hand side alone is formed again, with the factors of the fields written since
+    D = len(n)
+    fd = cm.field_desc(D, capi.CENTER, [(capi.BC_DIRC, capi.BC_DIRC)] * D, ext=1)
+    mesh = cm.mesh_uniform([m + 1 for m in n])
+    p, K, f = (api.CartesianField(mesh, fd, ctx) for _ in range(3))
+    K.assign(1.5 + 0.0 * f)
+    f.assign(0.0 * K + 1.0)
+
+    def eq(e):
+        t = 2.0 * e
+        for d in range(D):
+            t = t - 1e-3 * api.d1(api.d1IntpCenterToCorner(K, d) * api.d1(e, d), d)
+        return api.Eq(t, f)
+    s = api.EqnSolveHandler(eq, p, api.StructSolverParams(tol=1e-8, maxIter=30, precision="mixed", staticMat=True))
+    assert s.solve().converged and s.solve().converged
+    f.assign(0.0 * K + 2.0)
+    assert s.solve().converged
+    a = K.download()
+    a[tuple(m // 2 for m in reversed(n))] = np.inf
+    K.upload(a)
+    st = s.solve()
+    assert not st.converged and np.isnan(st.relerr)
