@@ -5,11 +5,11 @@
 // What bounds such levels is latency: a half sweep of a few thousand cells is a few passes of a CTA, each a
 // chain of five shared-memory reads, five dependent operations and a barrier (about 200 cycles), where a
 // launch or a strip's march over the level's rows takes microseconds.  So cells are spread over all threads,
-// one barrier per half sweep among the warps that a level needs.  A thread keeps its cells' places and inverse
-// centres for all half sweeps of a level, and the levels' geometry comes laid out by the host in one piece.  The
+// one barrier per half sweep among the warps that a level needs.  A thread forms its cells' places and inverse
+// centres once for all half sweeps of a level, and the levels' geometry comes laid out by the host in one piece.  The
 // code stays short (loops are not unrolled): a launch finds it cold in the instruction caches, and fetching an
-// unrolled version took a third of the time.  Levels are framed by a ring of zeros, so that a neighbour that does not exist costs no test (its
-// coefficient times 0 leaves the sum as it is).  A half sweep's warp takes 16 cells of one row and 16 of the
+// unrolled version took a third of the time.  Levels are framed by a ring of zeros, so that a neighbour that does not
+// exist costs no test (its coefficient times 0 leaves the sum as it is).  A half sweep's warp takes 16 cells of one row and 16 of the
 // next, whose colours alternate, so that its shared-memory accesses fall into distinct banks.
 //
 // The per-cell arithmetic is the chunked kernels' in their operation order (bit-identical iterates).  Measured,
@@ -35,7 +35,8 @@ __device__ __forceinline__ void small_sync(int warps, int id) {
 }
 static_assert(MG_BOTTOM_LEVELS <= 15, "a named barrier per level");
 
-// One level in one thread's registers.  A warp share is 32 column pairs: 16 of two rows, or 8 of four or 4 of eight
+// One thread's part of a level.  Its places and inverse centres are indexed in loops that stay rolled, so they lie in
+// local memory (64 bytes a thread, in the L1): read once per half sweep, ahead of the shared memory.  A warp share is 32 column pairs: 16 of two rows, or 8 of four or 4 of eight
 // where the rows are short; a thread holds up to MG_SMALL_SHARES pairs (the cells of colour 0 and 1 next to each
 // other).  A level of fewer shares than warps is run by the first `act` warps alone, the others go on to where
 // the next larger level needs them again.

@@ -186,6 +186,7 @@ __device__ __forceinline__ void strip_down(const LvlDev& L, const LvlDev& Lc, co
     float* bc = Lc.b32;
     float* xc = Lc.x32;
     const int cn0 = Lc.n[0];
+    const bool adjoint = L.adjoint;
     const bool own_e = S.ge >= S.i0 && S.ge < S.i1, own_o = S.ge + 1 >= S.i0 && S.ge + 1 < S.i1;
     // (children beyond the level's faces are left out of the restriction, also where it is periodic)
     const bool ein = (unsigned) S.ge < (unsigned) S.n0, oin = (unsigned) (S.ge + 1) < (unsigned) S.n0;
@@ -232,7 +233,7 @@ __device__ __forceinline__ void strip_down(const LvlDev& L, const LvlDev& Lc, co
                 pa = __fadd_rn(re, ro);
             } else if (own_e && r - 1 >= S.j0 && r - 1 < S.j1) {
                 // average over the children that exist: 4, 2 or 1 (adjoint: as if all did)
-                const float sc = (r < S.n1 || L.adjoint ? 0.5f : 1.f) * (oin || L.adjoint ? 0.5f : 1.f);
+                const float sc = (r < S.n1 || adjoint ? 0.5f : 1.f) * (oin || adjoint ? 0.5f : 1.f);
                 const long long cc = (long long) (r >> 1) * cn0 + (S.ge >> 1);
                 bc[cc] = __fmul_rn(__fadd_rn(__fadd_rn(pa, re), ro), sc);
                 xc[cc] = 0.f;

@@ -145,6 +145,7 @@ __device__ __forceinline__ void vol_down(const LvlDev& L, const LvlDev& Lc, cons
     const long long sy = T.n0, sz = (long long) T.n0 * T.n1;
     const float* bg = L.b32 + T.ge + sy * T.y0;
     float* xg = L.r32 + T.ge + sy * T.y0;
+    const bool adjoint = L.adjoint;
     const bool own_e = T.ge >= T.i0 && T.ge < T.i1, own_o = T.ge + 1 >= T.i0 && T.ge + 1 < T.i1;
     bool own_r[2];
     for (int r = 0; r < 2; ++r) own_r[r] = T.y0 + r >= T.j0 && T.y0 + r < T.j1;
@@ -224,7 +225,7 @@ __device__ __forceinline__ void vol_down(const LvlDev& L, const LvlDev& Lc, cons
             const float acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(pa, res[0][0]), res[0][1]), res[1][0]), res[1][1]);
             if (own_e && own_r[0] && p - 1 >= T.k0 && p - 1 < T.k1) {
                 // average over the children that exist: 8, 4, 2 or 1 (adjoint: as if all did)
-                const float sc = L.adjoint ? 0.125f : (p < T.n2 ? 0.5f : 1.f) * (T.okr[1] ? 0.5f : 1.f) * (T.oko ? 0.5f : 1.f);
+                const float sc = adjoint ? 0.125f : (p < T.n2 ? 0.5f : 1.f) * (T.okr[1] ? 0.5f : 1.f) * (T.oko ? 0.5f : 1.f);
                 const long long cc = (T.ge >> 1) + (long long) Lc.n[0] * ((T.y0 >> 1) + (long long) Lc.n[1] * (p >> 1));
                 Lc.b32[cc] = __fmul_rn(acc, sc);
                 Lc.x32[cc] = 0.f;

@@ -118,6 +118,9 @@ struct MGSystem {
     // cells instead.  Measured, 2D with 1100, 3072, 6400, 9216 cells: 2048^2 solve (a level of 64^2) 3.09, 3.09,
     // 3.01, 3.01 ms, a served mix of 24 requests 190, 180, 186, 187 ms (levels of 70^2 to 90^2 are quicker as
     // strips); 3D with 600, 4096, 8000: 256^3 (16^3) 8.88, 8.77, 8.77 ms.
+    // What the bounds stand for on any problem: a level in the CTA takes its cells in passes of 2048 per half sweep, so its
+    // time grows with them, while two launches of strips take about 20 us for any level up to some 10^5 cells.  The two
+    // are even between 64^2 and 70^2 cells (64^2 and all below it 27 us in the CTA; strips 20 us for 64^2 alone).
     long long small_max2 = 4352, small_max3 = 4096;
     std::vector<int> small_host;
     std::vector<SmProblem> small_probs;  // laid out for the kernel, in small_host's order
