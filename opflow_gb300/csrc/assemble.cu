@@ -600,6 +600,7 @@ static bool inner_tape(const AsmPlan& plan, bool coef, bool hoist, Tape* T) {
     std::set<int> factors;
     auto num = [&] { const int v = nums.back(); nums.pop_back(); return v; };
     for (const PInstr& in : plan.prog) {
+        if (coef && T->too_long()) return false;  // (every value reaches a coefficient or the right-hand side)
         switch (in.op) {
             case Q_LOADS: nums.push_back(T->load(in.slot, P.leaves[in.slot], in.off)); break;
             case Q_LOADU: {
@@ -690,11 +691,13 @@ static bool inner_tape(const AsmPlan& plan, bool coef, bool hoist, Tape* T) {
             const int c = r.c.count(q) ? r.c.at(q) : T->cst(0.0);
             T->out(T_COEF, q, c);
             // (a factor is looked at beside the first coefficient it goes into: none is kept longer for it)
-            for (size_t k = 0; k < left.size();) {
-                if (!T->uses(c, left[k])) { ++k; continue; }
-                look_at(left[k]);
-                left.erase(left.begin() + k);
+            const std::vector<char> in = T->formed_from(c);
+            std::vector<int> later;
+            for (int s : left) {
+                if (s <= c && in[s]) look_at(s);
+                else later.push_back(s);
             }
+            left.swap(later);
         }
     for (int s : left) look_at(s);
     for (int d = 0; d < 3; ++d)
@@ -703,8 +706,12 @@ static bool inner_tape(const AsmPlan& plan, bool coef, bool hoist, Tape* T) {
     return true;
 }
 
-// Cells of the inner box from which its program is run apart from the shell's (below that one launch for both).
-constexpr long long ASM_TAPE_CELLS = 4096;
+// Cells of the inner box from which its program is run apart from the shell's (below that one launch of the general
+// program for both): of the right-hand side alone, and of the coefficients too, whose larger program takes the host longer
+// (60 us for a 2D flux form, 200 us for a sum of eight) than the general program takes fewer cells.  A whole assembly
+// by one / the other, coefficients read back: 2D flux form, 80 x 70 cells 369 / 312 us, 182^2 473 / 426, 256^2 701 / 642,
+// 400^2 1080 / 1128; sum of eight, 256^2 1351 / 1307, 400^2 1822 / 2529, 50^3 2368 / 2492.
+constexpr long long ASM_TAPE_CELLS_RHS = 4096, ASM_TAPE_CELLS = 65536;
 
 // ======================================================================== host structural evaluation
 // Key order of the middle cell's StencilPad (fake_map insertion order): the recursion of the
@@ -925,7 +932,7 @@ int asm_run(opflow_ctx ctx, AsmPlan* plan, double* coef, double* rhs) {
     Tape tape;
     bool taped = false;
     const bool hoist = in.count() >= 32768;
-    if (!plain && !pinned && in.count() >= ASM_TAPE_CELLS) taped = inner_tape(*plan, coef != nullptr, hoist, &tape) && tape.finish(in, hoist);
+    if (!plain && !pinned && in.count() >= (coef ? ASM_TAPE_CELLS : ASM_TAPE_CELLS_RHS)) taped = inner_tape(*plan, coef != nullptr, hoist, &tape) && tape.finish(in, hoist);
     int rc = OPFLOW_OK;
     if (plain) {
         const int nx = in.hi[0] - in.lo[0], rows = (in.hi[1] - in.lo[1]) * (in.hi[2] - in.lo[2]);

@@ -38,19 +38,37 @@ static long long bits_of(double v) {
     return b;
 }
 
+unsigned long long Tape::hash(const Node& n) {
+    unsigned long long h = (unsigned long long) bits_of(n.v) ^ (unsigned long long) n.lin * 0x9E3779B97F4A7C15ull;
+    h = (h ^ (h >> 32)) * 0xBF58476D1CE4E5B9ull + ((unsigned long long) n.op << 40 | (unsigned long long) n.slot << 48);
+    h = (h ^ (unsigned) n.a ^ (unsigned long long) (unsigned) n.b << 20 ^ (unsigned long long) (unsigned) n.c << 40) * 0x94D049BB133111EBull;
+    return h ^ (h >> 31);
+}
+
 int Tape::intern(const Node& n) {
-    const std::array<long long, 7> key{n.op, n.slot, n.a, n.b, n.c, n.lin, bits_of(n.v)};
-    auto it = index_.find(key);
-    if (it != index_.end()) return it->second;
+    if (2 * nodes_.size() >= index_.size()) {  // (at least half of it free)
+        index_.assign(std::max<size_t>(256, 2 * index_.size()), -1);
+        for (size_t q = 0; q < nodes_.size(); ++q) {
+            size_t at = hash(nodes_[q]) & (index_.size() - 1);
+            while (index_[at] >= 0) at = (at + 1) & (index_.size() - 1);
+            index_[at] = (int) q;
+        }
+    }
+    size_t at = hash(n) & (index_.size() - 1);
+    for (; index_[at] >= 0; at = (at + 1) & (index_.size() - 1)) {
+        const Node& m = nodes_[index_[at]];
+        if (m.op == n.op && m.slot == n.slot && m.a == n.a && m.b == n.b && m.c == n.c && m.lin == n.lin && bits_of(m.v) == bits_of(n.v)) return index_[at];
+    }
+    index_[at] = (int) nodes_.size();
     nodes_.push_back(n);
     per_cell_ += n.op != T_CONST && n.op != T_NEG && n.dep != 1 && n.dep != 2 && n.dep != 4;
-    return index_[key] = (int) nodes_.size() - 1;
+    return index_[at];
 }
 bool Tape::too_long() const { return per_cell_ > TP_CODE; }
 
 int Tape::cst(double v) { return intern(Node{T_CONST, 0, -1, -1, -1, 0, v, 0}); }
 int Tape::load(int slot, const FieldView& f, const int* off) {
-    return intern(Node{T_LOAD, slot, -1, -1, -1, off[0] + off[1] * (long long) f.sy + off[2] * (long long) f.sz, 0., 8});
+    return intern(Node{T_LOAD, slot, -1, -1, -1, off[0] + off[1] * (long long) f.sy + off[2] * (long long) f.sz, 0., 8 | (256 << slot)});
 }
 int Tape::pos(int op, int d, int o) { return intern(Node{op, d, -1, -1, -1, o, 0., 1 << d}); }
 
@@ -65,27 +83,13 @@ int Tape::direction(int id) const {
     return d == 1 ? 0 : d == 2 ? 1 : d == 4 ? 2 : -1;
 }
 
-bool Tape::uses(int id, int operand) const {
-    if (id < operand) return false;  // (operands come first)
-    std::vector<char> from(id + 1 - operand, 0);
-    from[0] = 1;
-    for (int q = operand + 1; q <= id; ++q)
-        for (int o : {nodes_[q].a, nodes_[q].b, nodes_[q].c})
-            if (o >= operand && from[o - operand]) from[q - operand] = 1;
-    return from[id - operand];
-}
-
-unsigned Tape::fields(int id) const {
+std::vector<char> Tape::formed_from(int id) const {
     std::vector<char> in(id + 1, 0);
     in[id] = 1;
-    unsigned f = 0;
-    for (int q = id; q >= 0; --q) {
-        if (!in[q]) continue;
-        if (nodes_[q].op == T_LOAD) f |= 1u << nodes_[q].slot;
+    for (int q = id; q >= 0; --q)  // (operands come first)
         for (int o : {nodes_[q].a, nodes_[q].b, nodes_[q].c})
-            if (o >= 0) in[o] = 1;
-    }
-    return f;
+            if (o >= 0 && in[q]) in[o] = 1;
+    return in;
 }
 
 int Tape::node(int op, int slot, int a, int b, int c) {

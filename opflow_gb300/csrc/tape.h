@@ -59,8 +59,8 @@ public:
     int direction(int id) const;  // the direction whose mesh positions alone a value depends on, -1: none or several
     void out(int op, int slot, int id) { outs_.push_back({op, slot, id}); }
     void form(int id) { outs_.push_back({T_CONST, 0, id}); }  // here in the program, read by a later one
-    bool uses(int id, int operand) const;                     // whether id is, or is formed from, operand
-    unsigned fields(int id) const;                            // the leaf slots that id is formed from, a bit each
+    std::vector<char> formed_from(int id) const;              // per value up to id: whether id is it or is formed from it
+    unsigned fields(int id) const { return (unsigned) nodes_[id].dep >> 8; }  // the leaf slots that id is formed from, a bit each
     // Whether the values formed so far, each of them read by the program's result, are already more than the kernel
     // takes (constants, negations and values of one direction left out: they may go elsewhere); finish() is then false.
     bool too_long() const;
@@ -74,14 +74,15 @@ public:
     void release(opflow_ctx ctx);
 
 private:
-    struct Node { int op, slot, a, b, c; long long lin; double v; int dep; };  // dep: bit d: X or DX along d; bit 3: a field
+    struct Node { int op, slot, a, b, c; long long lin; double v; int dep; };  // dep: bit d: X or DX along d; bit 3: a field; bit 8 + s: leaf s
     struct Out { int op, slot, id; };
     struct Program { std::vector<TInstr> code; int slots = 0; };
+    static unsigned long long hash(const Node& n);
     int intern(const Node& n);
     bool emit(const std::vector<Out>& outs, const std::vector<int>& tab, Program* P);
     int const_at(const std::vector<double>& block);
     std::vector<Node> nodes_;
-    std::map<std::array<long long, 7>, int> index_;
+    std::vector<int> index_;  // the values by their hash (open addressing, -1: free)
     std::vector<Out> outs_;
     std::vector<double> consts_;
     std::map<std::vector<long long>, int> const_index_;
