@@ -133,7 +133,7 @@ def test_assembled_inner_cells_match_the_oracle(ctx, n, stretched, bc, pin):
     assert np.array_equal(rhs, want_rhs)
 
 
-@pytest.mark.parametrize("n", [[80, 70], [40, 33, 20]])
+@pytest.mark.parametrize("n", [[80, 70], [300, 260], [40, 33, 20], [50, 44, 42]])
 @pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
 def test_infinite_and_nan_coefficients_reach_the_right_hand_side(ctx, n, bad):
     # the bias of a pad is always there, and 0 times an infinite factor is NaN
@@ -190,3 +190,10 @@ def test_coefficients_that_become_infinite_reach_a_kept_matrix_s_right_hand_side
     K.upload(a)
     st = s.solve()
     assert not st.converged and np.isnan(st.relerr)
+
+
+@pytest.mark.parametrize("n,stretched", [([300, 260], False), ([300, 260], True), ([50, 44, 42], False), ([50, 44, 42], True), ([258, 258], False), ([256, 259], True)])
+@pytest.mark.parametrize("bc,pin", [("neum", True), ("neum", False), ("dirc", False)])
+def test_assembled_inner_cells_of_larger_boxes(ctx, n, stretched, bc, pin):
+    # (from 65536 inner cells the coefficients come from the scalar program: 256 x 256 of 258 x 258, 254 x 257 of 256 x 259)
+    test_assembled_inner_cells_match_the_oracle(ctx, n, stretched, bc, pin)
